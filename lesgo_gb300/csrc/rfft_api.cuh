@@ -1,0 +1,23 @@
+// Launchers of the register-transform passes (rfft_pass.cuh),
+// defined in rfft_launch.cuh and instantiated in translation units of their
+// own.  The length must be one of the lists of rfft_pass.cuh.
+#pragma once
+#include "rfft_pass.cuh"
+
+namespace lesgo {
+
+template <typename A, class Src> void rx_fwd(const RxGeom<A>& g, const Src& src, cplx<A>* out, cudaStream_t st);
+template <typename A, class Dst> void rx_inv(const RxGeom<A>& g, const cplx<A>* in, const Dst& dst, cudaStream_t st);
+template <typename A> void rx_fwd21(const RxGeom<A>& g, const SrcLagrange<A>& src, cplx<A>* out, cudaStream_t st);
+template <typename A> void rx_inv42(const RxGeom<A>& g, const cplx<A>* in, const DstLagrange<A>& dst, cudaStream_t st);
+
+enum RyKind { RY_FILT, RY_DIV, RY_PAD, RY_UNPAD, RY_TEST1, RY_TEST2 };
+// ny rows (the small grid's count) of nf fields, nlev planes
+template <typename A>
+void ry_pass(RyKind kind, const RyArgs<A, cplx<A>, cplx<A>>& a, int ny, int nlev, int nf, cudaStream_t st);
+template <typename A>
+void ry_spec(const RyArgs<A, cplx<A>, double2>& a, int ny, int nlev, int nf, cudaStream_t st);
+template <typename A>
+void ry_phys(bool grad, const RyArgs<A, double2, cplx<A>>& a, int ny, int nlev, cudaStream_t st);
+
+}  // namespace lesgo

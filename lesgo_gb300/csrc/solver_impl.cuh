@@ -6,7 +6,9 @@
 // C ABI (solver.cu) reaches them through make_solver_*.
 #pragma once
 #include "lesgo_gpu.h"
+#include "launch_util.hpp"
 #include "kernels.cuh"
+#include "rfft_api.cuh"
 #include "convec_rows.cuh"
 #include "tc_dft.cuh"
 #include "restart_io.hpp"
@@ -27,19 +29,6 @@
 #include <vector>
 
 namespace lesgo {
-
-struct Error : std::runtime_error {
-  int code;
-  Error(int c, const std::string& m) : std::runtime_error(m), code(c) {}
-};
-
-#define CK(x)                                                                                 \
-  do {                                                                                        \
-    cudaError_t e_ = (x);                                                                     \
-    if (e_ != cudaSuccess)                                                                    \
-      throw Error(e_ == cudaErrorMemoryAllocation ? LESGO_ERR_NOMEM : LESGO_ERR_CUDA,         \
-                  std::string(#x) + ": " + cudaGetErrorString(e_));                           \
-  } while (0)
 
 static const long double kPiL = 3.141592653589793238462643383279502884L;
 static const double kPi = 3.1415926535897932384626433;   // param.f90:94
@@ -201,25 +190,6 @@ static bool convec_rows_enabled(int precision) {
   return precision != LESGO_FP64;
 }
 
-// A kernel's dynamic shared-memory limit (cudaFuncAttributeMaxDynamicSharedMemorySize)
-// belongs to the function, not to a launch, and a replayed CUDA graph
-// launches its kernel nodes against the value current at replay.  Handles
-// of different grids share the kernel instances, so a handle that set a
-// smaller limit than another handle's captured node needs would break that
-// node's replay.  The limit is therefore only ever raised, per device,
-// under a lock (handles may live on several host threads).
-static void raise_smem_limit(const void* kern, size_t bytes) {
-  static std::mutex mu;
-  static std::map<std::pair<int, const void*>, size_t> limit;
-  int dev = 0;
-  CK(cudaGetDevice(&dev));
-  std::lock_guard<std::mutex> lk(mu);
-  size_t& cur = limit[{dev, kern}];
-  if (bytes <= cur) return;
-  CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-  cur = bytes;
-}
-
 // Device bytes of a handle (the admission footprint of a batch).
 static long long footprint_bytes(const Derived& d, int cap) {
   const long long rs = d.p.precision == LESGO_MIXED ? 4 : 8;
@@ -247,6 +217,26 @@ template <> struct HostCvt<df64> {
     return df64{h, (float)(v - (long double)h)};
   }
 };
+
+// Which arithmetic, row loaders and row epilogues have passes with the
+// transforms in registers (rfft_api.cuh).
+template <typename A> constexpr bool kRf = std::is_same<A, float>::value;
+template <class S> constexpr bool kRxSrc = false;
+template <typename R> constexpr bool kRxSrc<SrcFields<R, 1>> = true;
+template <typename R> constexpr bool kRxSrc<SrcFields<R, 2>> = true;
+template <typename R> constexpr bool kRxSrc<SrcFields<R, 3>> = true;
+template <typename R> constexpr bool kRxSrc<SrcFields<R, 5>> = true;
+template <typename R, bool VO> constexpr bool kRxSrc<SrcVort<R, VO>> = true;
+template <typename R> constexpr bool kRxSrc<SrcLagrange<R>> = true;
+template <class D> constexpr bool kRxDst = false;
+template <typename R> constexpr bool kRxDst<DstFields<R, 1>> = true;
+template <typename R> constexpr bool kRxDst<DstFields<R, 2>> = true;
+template <typename R> constexpr bool kRxDst<DstFields<R, 3>> = true;
+template <typename R> constexpr bool kRxDst<DstFields<R, 9>> = true;
+template <typename R, int W> constexpr bool kRxDst<DstDiv<R, W>> = true;
+template <typename R, bool F> constexpr bool kRxDst<DstConvec<R, F>> = true;
+template <typename R, bool F> constexpr bool kRxDst<DstPress<R, F>> = true;
+template <typename R> constexpr bool kRxDst<DstLagrange<R>> = true;
 
 // R: the fields' storage and pointwise arithmetic; A: the transforms'
 // arithmetic and spectral storage (R itself, or df64 for FP64 fields).
@@ -324,6 +314,8 @@ class Solver : public SolverBase {
     if (const char* e = std::getenv("LESGO_YSHORTCUT")) yshort_ = std::strcmp(e, "0") != 0;
     if (const char* e = std::getenv("LESGO_THOMAS"))
       thomas_mode_ = std::strcmp(e, "seq") == 0 ? 1 : std::strcmp(e, "seg") == 0 ? 2 : 0;
+    // LESGO_RFFT=0: every pass on the run-time radix stages of fft_core.cuh
+    if (const char* e = std::getenv("LESGO_RFFT")) rf_ = std::strcmp(e, "0") != 0;
     use_graphs_ = graphs_allowed_;
     build_tables();
     // x-direction forward transforms as tensor-core GEMMs (FP32 transforms,
@@ -452,8 +444,7 @@ class Solver : public SolverBase {
     const R sc = (R)(1.0 / ((double)d_.nx * d_.ny));
     SrcFields<R, 1> src{{F_[f]}, sc, 1, 1, d_.ld, kp_.plane, imf(d_.nz)};
     xfwd<1>(src, d_.nx, d_.ny, d_.nz, specA_, px_);
-    ypass_lin<1, 3, true, true, T2, T2>(specA_, 0, 1, d_.nz, d_.ny, specB_, d_.ny, d_.nz, 1, ROW_SAME,
-                                        {{MUL_ONE}, {MUL_IKX}, {MUL_IKY}});
+    y_pass(RY_FILT, specA_, specB_, d_.nz, 1, "ypass");
     DstFields<R, 3> dst{{F_[f], F_[fx], F_[fy]}, 1, 1, d_.ld, kp_.plane, imf(d_.nz)};
     xinv<3>(dst, specB_, d_.nx, d_.ny, d_.nz, px_);
   }
@@ -519,25 +510,21 @@ class Solver : public SolverBase {
       SrcFields<R, 5> src{{F_[LESGO_TXX], F_[LESGO_TXY], F_[LESGO_TYY], F_[LESGO_TXZ], F_[LESGO_TYZ]}, sc, 1, 1, d_.ld,
                           kp_.plane, im};
       xfwd<5>(src, d_.nx, d_.ny, d_.nz, specA_, px_, "divstress.xfwd");
-      ypass_lin<5, 3, true, true, T2, T2>(specA_, 0, 1, d_.nz, d_.ny, specB_, d_.ny, d_.nz, 1, ROW_SAME,
-                                          {{MUL_IKX, MUL_IKY, 0, 0, 0}, {0, MUL_IKX, MUL_IKY, 0, 0}, {0, 0, 0, MUL_IKX, MUL_IKY}},
-                                          "divstress.ypass");
+      y_pass(RY_DIV, specA_, specB_, d_.nz, 3, "divstress.ypass");
       DstDiv<R, 3> dst{F_[LESGO_DIVTX], F_[LESGO_DIVTY], F_[LESGO_DIVTZ], F_[LESGO_TXZ], F_[LESGO_TYZ], F_[LESGO_TZZ],
                        idz, d_.ld, d_.nz, kp_.plane, im};
       xinv<3>(dst, specB_, d_.nx, d_.ny, d_.nz, px_, "divstress.xinv", 6);
     } else if (which == 1) {
       SrcFields<R, 3> src{{F_[LESGO_TXX], F_[LESGO_TXY], F_[LESGO_TYY]}, sc, 1, 1, d_.ld, kp_.plane, im};
       xfwd<3>(src, d_.nx, d_.ny, d_.nz, specA_, px_);
-      ypass_lin<3, 2, true, true, T2, T2>(specA_, 0, 1, d_.nz, d_.ny, specB_, d_.ny, d_.nz, 1, ROW_SAME,
-                                          {{MUL_IKX, MUL_IKY, 0}, {0, MUL_IKX, MUL_IKY}});
+      y_pass(RY_DIV, specA_, specB_, d_.nz, 2, "ypass");
       DstDiv<R, 1> dst{F_[LESGO_DIVTX], F_[LESGO_DIVTY], F_[LESGO_DIVTZ], F_[LESGO_TXZ], F_[LESGO_TYZ], F_[LESGO_TZZ],
                        idz, d_.ld, d_.nz, kp_.plane, im};
       xinv<2>(dst, specB_, d_.nx, d_.ny, d_.nz, px_);
     } else {
       SrcFields<R, 2> src{{F_[LESGO_TXZ], F_[LESGO_TYZ]}, sc, 1, 1, d_.ld, kp_.plane, im};
       xfwd<2>(src, d_.nx, d_.ny, d_.nz, specA_, px_);
-      ypass_lin<2, 1, true, true, T2, T2>(specA_, 0, 1, d_.nz, d_.ny, specB_, d_.ny, d_.nz, 1, ROW_SAME,
-                                          {{MUL_IKX, MUL_IKY}});
+      y_pass(RY_DIV, specA_, specB_, d_.nz, 1, "ypass");
       DstDiv<R, 2> dst{F_[LESGO_DIVTX], F_[LESGO_DIVTY], F_[LESGO_DIVTZ], F_[LESGO_TXZ], F_[LESGO_TYZ], F_[LESGO_TZZ],
                        idz, d_.ld, d_.nz, kp_.plane, im};
       xinv<1>(dst, specB_, d_.nx, d_.ny, d_.nz, px_);
@@ -1503,8 +1490,7 @@ class Solver : public SolverBase {
                         kp_.plane, im};
     // into the convective term's spectra, which reuses them (convec_part1)
     xfwd<3>(src, d_.nx, d_.ny, d_.nz, cvA_, px_, "filt_da.xfwd");
-    ypass_lin<1, 3, true, true, T2, T2>(cvA_, 0, 1, d_.nz, d_.ny, specB_, d_.ny, d_.nz, 3, ROW_SAME,
-                                        {{MUL_ONE}, {MUL_IKX}, {MUL_IKY}}, "filt_da.ypass");
+    y_pass(RY_FILT, cvA_, specB_, d_.nz, 3, "filt_da.ypass");
     DstFields<R, 9> dst{{F_[LESGO_U], F_[LESGO_DUDX], F_[LESGO_DUDY], F_[LESGO_V], F_[LESGO_DVDX], F_[LESGO_DVDY],
                          F_[LESGO_W], F_[LESGO_DWDX], F_[LESGO_DWDY]}, 1, 1, d_.ld, kp_.plane, im};
     xinv<9>(dst, specB_, d_.nx, d_.ny, d_.nz, px_, "filt_da.xinv");
@@ -1632,6 +1618,18 @@ class Solver : public SolverBase {
     return p;
   }
 
+  // Twiddles of the register transforms of length r1 r2, [k1][n2].
+  T2* rf_table(int r1, int r2) {
+    std::vector<T2> t;
+    t.reserve((size_t)r1 * r2);
+    for (int k1 = 0; k1 < r1; ++k1)
+      for (int n2 = 0; n2 < r2; ++n2) {
+        const long double a = -2.0L * kPiL * (long double)(k1 * n2) / (long double)(r1 * r2);
+        t.push_back(mkc(HostCvt<A>::from(cosl(a)), HostCvt<A>::from(sinl(a))));
+      }
+    return upload_vec(t);
+  }
+
   // Thomas pivots of every (kx, ky) column (tridag_array.f90:166-246): they
   // depend only on the wavenumbers and dz, so they are formed once in FP64.
   void build_thomas_pivots() {
@@ -1673,6 +1671,14 @@ class Solver : public SolverBase {
     py_ = make_plan(d_.ny);
     pxb_ = make_plan(d_.nx2 / 2);
     pyb_ = make_plan(d_.ny2);
+    if (kRf<A> && rf_) {
+      int r1 = 0, r2 = 0;
+      if (rx_factors(d_.nx / 2, &r1, &r2)) rx_tw_ = rf_table(r1, r2);
+      if (yshort_ && ry_factors(d_.ny, &r1, &r2)) {
+        ry_twn_ = rf_table(r1, r2);
+        ry_twm_ = rf_table(r1, 3 * r2 / 2);
+      }
+    }
     // wavenumbers (fft.f90:130-160) for kx < nx/2 and every ky row
     const int ny = d_.ny, lh = d_.lh;
     std::vector<double> kx(d_.K), ky(ny);
@@ -1745,6 +1751,21 @@ class Solver : public SolverBase {
         return;
       }
     }
+    if constexpr (kRf<A> && kRxSrc<Src>) {
+      if (rx_tw_ && M == d_.nx) {
+        const RxGeom<A> rg = rx_geom(NF, nyrows, nli);
+        pre();
+        if constexpr (std::is_same<Src, SrcLagrange<R>>::value) {
+          rx_fwd21(rg, src, out, st_);
+        } else {
+          Src h = src;
+          halve(h);   // the split's factor 1/2
+          rx_fwd(rg, h, out, st_);
+        }
+        post(tag, (double)rg.nrows * ((double)in_fields * M * sizeof(R) + (double)NF * d_.K * sizeof(T2)));
+        return;
+      }
+    }
     XfGeom g;
     g.M = M; g.K = d_.K; g.nyrows = nyrows; g.nrows = nyrows * nli * kp_.ninst; g.ls = M / 2 + 1;
     const int target = xtarget_;
@@ -1760,6 +1781,18 @@ class Solver : public SolverBase {
     kern<<<(g.nrows + g.rpc - 1) / g.rpc, 256, smem, st_>>>(g, plan, src, out);
     post(tag, (double)g.nrows * ((double)in_fields * M * sizeof(R) + (double)NF * g.K * sizeof(T2)));
   }
+
+  RxGeom<A> rx_geom(int nf, int nyrows, int nli) const {
+    RxGeom<A> g{};
+    g.N = d_.K; g.nf = nf; g.nyrows = nyrows; g.nrows = nyrows * nli * kp_.ninst;
+    g.fny = FastDiv((unsigned)nyrows);
+    g.fs = (long long)g.nrows * g.N;
+    g.kz0 = g.kz1 = g.N;
+    g.tw = rx_tw_; g.rtw = px_.rtw;
+    return g;
+  }
+  template <int NF> static void halve(SrcFields<R, NF>& s) { s.scale = s.isc ? (R)0.5 : (R)0.5 * s.scale; }
+  template <bool VO> static void halve(SrcVort<R, VO>& s) { s.c = (R)0.5 * s.c; }
 
   // The same transform as a tensor-core GEMM (k_xdft_tc): tiles of 128 rows,
   // one persistent block per SM (its shared memory holds W).
@@ -1795,6 +1828,21 @@ class Solver : public SolverBase {
   template <int NF, class Dst>
   void xinv(const Dst& dst, const T2* in, int M, int nyrows, int nli, const FftPlan<A>& plan, const char* tag = "xinv",
             int out_fields = NF, int kz_even = -1, int kz_odd = -1) {
+    if constexpr (kRf<A> && kRxDst<Dst>) {
+      if (rx_tw_ && M == d_.nx) {
+        RxGeom<A> rg = rx_geom(NF, nyrows, nli);
+        pre();
+        if constexpr (std::is_same<Dst, DstLagrange<R>>::value) {
+          rg.kz0 = kz_even < 0 ? rg.N : std::min(kz_even, rg.N);
+          rg.kz1 = kz_odd < 0 ? rg.N : std::min(kz_odd, rg.N);
+          rx_inv42(rg, in, dst, st_);
+        } else {
+          rx_inv(rg, in, dst, st_);
+        }
+        post(tag, (double)rg.nrows * ((double)NF * d_.K * sizeof(T2) + (double)out_fields * M * sizeof(R)));
+        return;
+      }
+    }
     XiGeom g;
     g.M = M; g.K = d_.K; g.nyrows = nyrows; g.nrows = nyrows * nli * kp_.ninst; g.ls = M / 2 + 1;
     g.kz0 = kz_even < 0 ? g.K : std::min(kz_even, g.K);
@@ -1920,6 +1968,101 @@ class Solver : public SolverBase {
                   ((double)NIN * in_rows * sizeof(InT) + (double)NOUT * out_rows * sizeof(OutT)));
   }
 
+  // Arguments of a y pass with the transforms in registers: ngroups input
+  // fields of in_inst_levels planes per instance, as ypass_lin's.
+  template <typename InT, typename OutT>
+  RyArgs<A, InT, OutT> ry_args(const InT* in, int in_lev0, int in_levstride, int in_inst_levels, int in_rows, OutT* out,
+                               int out_rows, int nli) const {
+    RyArgs<A, InT, OutT> a{};
+    a.in = in; a.out = out;
+    a.in_fs = (long long)in_inst_levels * kp_.ninst * in_rows * d_.K;
+    a.out_fs = (long long)nli * kp_.ninst * out_rows * d_.K;
+    a.K = d_.K; a.lh = d_.lh;
+    a.nli = nli; a.in_inst_levels = in_inst_levels; a.in_lev0 = in_lev0; a.in_levstride = in_levstride;
+    a.fnli = FastDiv((unsigned)nli);
+    a.twn = ry_twn_; a.twm = ry_twm_;
+    a.kxw = kxw_; a.kyw = kyw_; a.G1 = G1_; a.G2 = G2_;
+    a.zero1 = kmax_g_[0] + 1; a.zero2 = kmax_g_[1] + 1;
+    return a;
+  }
+  // The y passes of the step: transforms in registers where ny is one of
+  // their lengths, else the run-time radix stages.
+  void y_pass(RyKind kind, const T2* in, T2* out, int nli, int nf, const char* tag) {
+    const int ny = d_.ny, ny2 = d_.ny2;
+    const int rin = kind == RY_UNPAD ? ny2 : ny, rout = kind == RY_PAD ? ny2 : ny;
+    if constexpr (kRf<A>) {
+      if (ry_twn_) {
+        const int nlev = nli * kp_.ninst;
+        RyArgs<A, T2, T2> a = ry_args(in, 0, 1, nli, rin, out, rout, nli);
+        const int ia[3] = {0, 1, 3}, ib[3] = {1, 2, 4};
+        for (int i = 0; i < 3; ++i) { a.ia[i] = ia[i]; a.ib[i] = ib[i]; }
+        pre();
+        ry_pass<A>(kind, a, ny, nlev, nf, st_);
+        const int no = kind == RY_FILT ? 3 : kind == RY_TEST2 ? 2 : 1;
+        const double ni = kind == RY_DIV ? (nf == 3 ? 5.0 / 3.0 : nf == 2 ? 1.5 : 2.0) : 1.0;
+        post(tag, (double)nf * nlev * d_.K * (ni * rin + no * rout) * sizeof(T2));
+        return;
+      }
+    }
+    switch (kind) {
+      case RY_FILT:
+        ypass_lin<1, 3, true, true, T2, T2>(in, 0, 1, nli, ny, out, ny, nli, nf, ROW_SAME, {{MUL_ONE}, {MUL_IKX}, {MUL_IKY}}, tag);
+        break;
+      case RY_DIV:
+        if (nf == 3)
+          ypass_lin<5, 3, true, true, T2, T2>(in, 0, 1, nli, ny, out, ny, nli, 1, ROW_SAME,
+                                              {{MUL_IKX, MUL_IKY, 0, 0, 0}, {0, MUL_IKX, MUL_IKY, 0, 0}, {0, 0, 0, MUL_IKX, MUL_IKY}}, tag);
+        else if (nf == 2)
+          ypass_lin<3, 2, true, true, T2, T2>(in, 0, 1, nli, ny, out, ny, nli, 1, ROW_SAME, {{MUL_IKX, MUL_IKY, 0}, {0, MUL_IKX, MUL_IKY}}, tag);
+        else
+          ypass_lin<2, 1, true, true, T2, T2>(in, 0, 1, nli, ny, out, ny, nli, 1, ROW_SAME, {{MUL_IKX, MUL_IKY}}, tag);
+        break;
+      case RY_PAD:
+        ypass_lin<1, 1, true, true, T2, T2>(in, 0, 1, nli, ny, out, ny2, nli, nf, ROW_PAD, {{MUL_ONE}}, tag);
+        break;
+      case RY_UNPAD:
+        ypass_lin<1, 1, true, true, T2, T2>(in, 0, 1, nli, ny2, out, ny, nli, nf, ROW_UNPAD, {{MUL_ONE}}, tag);
+        break;
+      case RY_TEST1:
+        ypass_lin<1, 1, true, true, T2, T2>(in, 0, 1, nli, ny, out, ny, nli, nf, ROW_SAME, {{MUL_G1}}, tag);
+        break;
+      case RY_TEST2:
+        // zero tiles are not written: the consumer does not read those modes
+        ypass_lin<1, 2, true, true, T2, T2>(in, 0, 1, nli, ny, out, ny, nli, nf, ROW_SAME, {{MUL_G1}, {MUL_G2}}, tag, false);
+        break;
+    }
+  }
+  // Forward only, in FP64 spectra (the pressure's right-hand sides).
+  void y_spec(const T2* in, double2* out, int nli, int nf, const char* tag) {
+    const int ny = d_.ny, nlev = nli * kp_.ninst;
+    if constexpr (kRf<A>) {
+      if (ry_twn_) {
+        pre();
+        ry_spec<A>(ry_args(in, 0, 1, nli, ny, out, ny, nli), ny, nlev, nf, st_);
+        post(tag, (double)nf * nlev * d_.K * ny * (sizeof(T2) + sizeof(double2)));
+        return;
+      }
+    }
+    ypass_lin<1, 1, true, false, T2, double2>(in, 0, 1, nli, ny, out, ny, nli, nf, ROW_SAME, {{MUL_ONE}}, tag);
+  }
+  // Inverse only, from the FP64 pressure spectra: p, or p, i kx p, i ky p.
+  void y_phys(bool grad, int lev0, int levstride, T2* out, int nli, const char* tag) {
+    const int ny = d_.ny, nlev = nli * kp_.ninst;
+    if constexpr (kRf<A>) {
+      if (ry_twn_) {
+        pre();
+        ry_phys<A>(grad, ry_args<double2, T2>(phat_, lev0, levstride, d_.nz + 1, ny, out, ny, nli), ny, nlev, st_);
+        post(tag, (double)nlev * d_.K * ny * (sizeof(double2) + (grad ? 3.0 : 1.0) * sizeof(T2)));
+        return;
+      }
+    }
+    if (grad)
+      ypass_lin<1, 3, false, true, double2, T2>(phat_, lev0, levstride, d_.nz + 1, ny, out, ny, nli, 1, ROW_SAME,
+                                                {{MUL_ONE}, {MUL_IKX}, {MUL_IKY}}, tag);
+    else
+      ypass_lin<1, 1, false, true, double2, T2>(phat_, lev0, levstride, d_.nz + 1, ny, out, ny, nli, 1, ROW_SAME, {{MUL_ONE}}, tag);
+  }
+
   // test filter (G_test) of plane `level` of two fields into two planes per
   // instance (out planes are `ostr` apart between instances)
   void filter_planes(const R* a, const R* b, int level, R* oa, R* ob, int nf, long long ostr) {
@@ -1928,7 +2071,7 @@ class Solver : public SolverBase {
     T2* outp = specC_ + 2 * pl_s * kp_.ninst;
     SrcFields<R, 2> src{{a, b}, (R)1, level, 1, d_.ld, kp_.plane, imf(1)};
     xfwd<2>(src, d_.nx, d_.ny, 1, in, px_, "wall_filter.xfwd");
-    ypass_lin<1, 1, true, true, T2, T2>(in, 0, 1, 1, d_.ny, outp, d_.ny, 1, 2, ROW_SAME, {{MUL_G1}}, "wall_filter.ypass");
+    y_pass(RY_TEST1, in, outp, 1, 2, "wall_filter.ypass");
     if (nf == 1) {
       DstFields<R, 1> dst{{oa}, 0, 1, d_.ld, 0, InstMap(1, ostr)};
       xinv<1>(dst, outp, d_.nx, d_.ny, 1, px_, "wall_filter.xinv");
@@ -1984,8 +2127,7 @@ class Solver : public SolverBase {
     // the 2-delta (even outputs) and 4-delta (odd) filtered spectra are zero
     // past the filters' cutoff columns: the y pass does not write those
     // tiles and the x inverse does not read those modes
-    ypass_lin<1, 2, true, true, T2, T2>(specA_, 0, 1, d_.nz, d_.ny, specB_, d_.ny, d_.nz, 21, ROW_SAME,
-                                        {{MUL_G1}, {MUL_G2}}, "lagrange.ypass", false);
+    y_pass(RY_TEST2, specA_, specB_, d_.nz, 21, "lagrange.ypass");
     DstLagrange<R> dst;
     dst.FLMi = Ftmp_[0]; dst.FMMi = Ftmp_[1]; dst.FQNi = Ftmp_[2]; dst.FNNi = Ftmp_[3];
     dst.FLM = F_[LESGO_F_LM]; dst.FMM = F_[LESGO_F_MM]; dst.FQN = F_[LESGO_F_QN]; dst.FNN = F_[LESGO_F_NN];
@@ -2027,8 +2169,7 @@ class Solver : public SolverBase {
                     F_[LESGO_DVDZ], F_[LESGO_DWDX], F_[LESGO_DWDY], c, d_.ld, d_.nz, kp_.lbc, kp_.ubc, kp_.plane, im};
       xfwd<6>(sv, d_.nx, d_.ny, d_.nz, cvA_, px_, "convec.xfwd", 9);
     }
-    ypass_lin<1, 1, true, true, T2, T2>(cvA_, 0, 1, d_.nz, d_.ny, cvB_, d_.ny2, d_.nz, 6, ROW_PAD, {{MUL_ONE}},
-                                        "convec.ypass_pad");
+    y_pass(RY_PAD, cvA_, cvB_, d_.nz, 6, "convec.ypass_pad");
     if (conv_rows_) {
       convec_rows(HostCvt<A>::from(1.0L / ((long double)d_.nx2 * d_.ny2)));
     } else {
@@ -2039,8 +2180,7 @@ class Solver : public SolverBase {
                         imb};
       xfwd<3>(sp, d_.nx2, d_.ny2, d_.nz, cvA_, pxb_, "convec.xfwd_big", 6);
     }
-    ypass_lin<1, 1, true, true, T2, T2>(cvA_, 0, 1, d_.nz, d_.ny2, cvB_, d_.ny, d_.nz, 3, ROW_UNPAD, {{MUL_ONE}},
-                                        "convec.ypass_unpad");
+    y_pass(RY_UNPAD, cvA_, cvB_, d_.nz, 3, "convec.ypass_unpad");
   }
   // The 3/2-grid x-rows of the convective term in one pass: the six padded
   // spectra of cvB_ in, the three products' x-spectra (nx/2 modes) into cvA_.
@@ -2155,11 +2295,9 @@ class Solver : public SolverBase {
     on_branch([&] {
       SrcFields<R, 1> sd{{F_[LESGO_DIVTZ]}, (R)c1, 1, nz - 1, d_.ld, kp_.plane, imf(2)};
       xfwd<1>(sd, d_.nx, ny, 2, specC_, px_, "press.xfwd_bc");
-      ypass_lin<1, 1, true, false, T2, double2>(specC_, 0, 1, 2, ny, hplane_, ny, 2, 1, ROW_SAME, {{MUL_ONE}},
-                                                "press.ypass_fwd_bc");
+      y_spec(specC_, hplane_, 2, 1, "press.ypass_fwd_bc");
     });
-    ypass_lin<1, 1, true, false, T2, double2>(specA_, 0, 1, nz, ny, hspec_, ny, nz, 3, ROW_SAME, {{MUL_ONE}},
-                                              "press.ypass_fwd");
+    y_spec(specA_, hspec_, nz, 3, "press.ypass_fwd");
     join(4);
     const long long vs = vol1_s_ * kp_.ninst;
     ThomasArgs ta;
@@ -2195,13 +2333,11 @@ class Solver : public SolverBase {
     // p at levels 0 and nz on the second stream
     fork(5);
     on_branch([&] {
-      ypass_lin<1, 1, false, true, double2, T2>(phat_, 0, nz, nz + 1, ny, specC_, ny, 2, 1, ROW_SAME, {{MUL_ONE}},
-                                                "press.ypass_inv_bc");
+      y_phys(false, 0, nz, specC_, 2, "press.ypass_inv_bc");
       DstFields<R, 1> d0{{F_[LESGO_P]}, 0, nz, d_.ld, kp_.plane, imf(2)};
       xinv<1>(d0, specC_, d_.nx, ny, 2, px_, "press.xinv_bc");
     });
-    ypass_lin<1, 3, false, true, double2, T2>(phat_, 1, 1, nz + 1, ny, specB_, ny, nz - 1, 1, ROW_SAME,
-                                              {{MUL_ONE}, {MUL_IKX}, {MUL_IKY}}, "press.ypass_inv");
+    y_phys(true, 1, 1, specB_, nz - 1, "press.ypass_inv");
     if (fused) {
       DstPress<R, true> dp{F_[LESGO_P], F_[LESGO_DPDX], F_[LESGO_DPDY], F_[LESGO_RHSX], F_[LESGO_RHSY], F_[LESGO_U],
                            F_[LESGO_V], sc_d_, d_.ld, kp_.plane, imf(nz - 1)};
@@ -2298,6 +2434,10 @@ class Solver : public SolverBase {
   double* staging_ = nullptr;
   long long staging_n_ = 0;
   FftPlan<A> px_{}, py_{}, pxb_{}, pyb_{};
+  // twiddles of the register transforms (null: the length is not one of
+  // theirs): x rows, y columns of ny and 3 ny / 2
+  bool rf_ = true;
+  T2 *rx_tw_ = nullptr, *ry_twn_ = nullptr, *ry_twm_ = nullptr;
   A *kxw_ = nullptr, *kyw_ = nullptr, *G1_ = nullptr, *G2_ = nullptr;
   int kmax_g_[2] = {1 << 30, 1 << 30};   // largest kx column with a nonzero G1 / G2 weight
   double *kxw64_ = nullptr, *kyw64_ = nullptr;
