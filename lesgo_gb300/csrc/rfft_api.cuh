@@ -1,8 +1,9 @@
-// Launchers of the register-transform passes (rfft_pass.cuh),
+// Launchers of the register-transform passes (rfft_pass.cuh, rfft_rows.cuh),
 // defined in rfft_launch.cuh and instantiated in translation units of their
 // own.  The length must be one of the lists of rfft_pass.cuh.
 #pragma once
 #include "rfft_pass.cuh"
+#include "rfft_rows.cuh"
 
 namespace lesgo {
 
@@ -19,5 +20,9 @@ template <typename A>
 void ry_spec(const RyArgs<A, cplx<A>, double2>& a, int ny, int nlev, int nf, cudaStream_t st);
 template <typename A>
 void ry_phys(bool grad, const RyArgs<A, double2, cplx<A>>& a, int ny, int nlev, cudaStream_t st);
+
+// cz = 0: chosen from the launch's waves
+template <typename A>
+void rx_rows(RxRowsGeom<A> g, int H, int ninst, const cplx<A>* in, cplx<A>* out, A c, cudaStream_t st);
 
 }  // namespace lesgo

@@ -88,4 +88,33 @@ void ry_phys(bool grad, const RyArgs<A, double2, cplx<A>>& a, int ny, int nlev, 
   });
 }
 
+template <typename A>
+void rx_rows(RxRowsGeom<A> g, int H, int ninst, const cplx<A>* in, cplx<A>* out, A c, cudaStream_t st) {
+  with_rxb(H, [&](auto len) {
+    constexpr int R1 = decltype(len)::R1, R2 = decltype(len)::R2, L = rows_lines<A, R1, R2>();
+    constexpr size_t smem = (L * rows_per_row<R1, R2>() + rows_besides<R1, R2>()) * sizeof(cplx<A>);
+    constexpr int threads = L * R1;
+    auto kern = k_rx_rows<A, R1, R2>;
+    smem_for(kern, smem);
+    // Levels per block: a block marches its chunk and about one level more
+    // (two and three fields of the levels around it), so the launch takes
+    // about (waves) x (chunk + 1) level times.
+    int per_sm = 0, nsm = 0, dev = 0;
+    CK(cudaGetDevice(&dev));
+    CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem));
+    const long long tiles = (long long)((g.ny2 + L - 1) / L) * ninst;
+    const long long slots = std::max(1LL, (long long)per_sm * nsm);
+    int best = 1;
+    long long best_t = -1;
+    for (int n = 1; n <= g.nz; ++n) {
+      const long long t = ((tiles * n + slots - 1) / slots) * ((g.nz + n - 1) / n + 1);
+      if (best_t < 0 || t < best_t) { best_t = t; best = n; }
+    }
+    g.cz = (g.nz + best - 1) / best;
+    kern<<<dim3((unsigned)((g.ny2 + L - 1) / L), (unsigned)((g.nz + g.cz - 1) / g.cz), (unsigned)ninst), threads, smem, st>>>(
+        g, in, out, c);
+  });
+}
+
 }  // namespace lesgo

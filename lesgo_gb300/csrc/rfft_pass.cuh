@@ -26,11 +26,16 @@ namespace lesgo {
 // real-transform split pairs mode k < N/2 with N - k.  y: ny = R1 R2 with R2
 // even and ny2 = 3 ny / 2 = R1 (3 R2 / 2): padding to the 3/2 grid and
 // truncation from it then only relabel the R2 or 3 R2 / 2 values that a
-// thread holds.
+// thread holds.  xb: complex length 3 nx / 4 of the 3/2 grid's rows; R1 is a
+// multiple of 3, so the padded modes are whole inputs of the first DFT, and
+// R2 <= 9 keeps the products' operands of one thread in registers.
 #define LESGO_RX_LENGTHS(X) \
   X(4, 4) X(3, 6) X(6, 4) X(8, 4) X(6, 6) X(8, 6) X(9, 6) X(8, 8) X(9, 8) X(12, 8) X(9, 12) X(16, 8)
 #define LESGO_RY_LENGTHS(X) \
   X(6, 4) X(8, 4) X(6, 6) X(8, 6) X(9, 6) X(8, 8) X(9, 8) X(12, 8) X(9, 12) X(16, 8) X(12, 12) X(16, 12) X(18, 12) X(16, 16)
+#define LESGO_RXB_LENGTHS(X) \
+  X(6, 4) X(9, 3) X(6, 6) X(6, 8) X(9, 6) X(9, 8) X(9, 9) X(12, 8) X(18, 6) X(18, 8) X(18, 9) X(24, 8)
+
 inline bool rx_factors(int n, int* r1, int* r2) {
 #define X(a, b) if (n == (a) * (b)) { *r1 = a; *r2 = b; return true; }
   LESGO_RX_LENGTHS(X)
@@ -40,6 +45,12 @@ inline bool rx_factors(int n, int* r1, int* r2) {
 inline bool ry_factors(int n, int* r1, int* r2) {
 #define X(a, b) if (n == (a) * (b)) { *r1 = a; *r2 = b; return true; }
   LESGO_RY_LENGTHS(X)
+#undef X
+  return false;
+}
+inline bool rxb_factors(int n, int* r1, int* r2) {
+#define X(a, b) if (n == (a) * (b)) { *r1 = a; *r2 = b; return true; }
+  LESGO_RXB_LENGTHS(X)
 #undef X
   return false;
 }
@@ -54,6 +65,12 @@ template <class F> void with_ry(int n, F&& fn) {
   LESGO_RY_LENGTHS(X)
 #undef X
 }
+template <class F> void with_rxb(int n, F&& fn) {
+#define X(a, b) if (n == (a) * (b)) { fn(Len<a, b>{}); return; }
+  LESGO_RXB_LENGTHS(X)
+#undef X
+}
+
 // ---------------------------------------------------------------------------
 // x passes
 // ---------------------------------------------------------------------------

@@ -1678,6 +1678,7 @@ class Solver : public SolverBase {
         ry_twn_ = rf_table(r1, r2);
         ry_twm_ = rf_table(r1, 3 * r2 / 2);
       }
+      if (conv_rows_ && rxb_factors(d_.nx2 / 2, &r1, &r2)) rxb_tw_ = rf_table(r1, r2);
     }
     // wavenumbers (fft.f90:130-160) for kx < nx/2 and every ky row
     const int ny = d_.ny, lh = d_.lh;
@@ -2185,6 +2186,18 @@ class Solver : public SolverBase {
   // The 3/2-grid x-rows of the convective term in one pass: the six padded
   // spectra of cvB_ in, the three products' x-spectra (nx/2 modes) into cvA_.
   void convec_rows(A cb) {
+    if constexpr (kRf<A>) {
+      if (rxb_tw_) {
+        RxRowsGeom<A> rg;
+        rg.ny2 = d_.ny2; rg.nz = d_.nz; rg.cz = 0; rg.err = err_ + 1;
+        rg.in_fs = rg.out_fs = vol1_b_ * kp_.ninst;
+        rg.tw = rxb_tw_; rg.rtw = pxb_.rtw;
+        pre();
+        rx_rows<A>(rg, d_.nx2 / 2, kp_.ninst, cvB_, cvA_, cb, st_);
+        post("convec.rows", 9.0 * vol1_b_ * kp_.ninst * sizeof(T2));
+        return;
+      }
+    }
     ConvRowsGeom g;
     g.M = d_.nx2; g.K = d_.K; g.ny2 = d_.ny2; g.nz = d_.nz; g.ls = d_.nx2 / 2 + 1;
     g.in_fs = vol1_b_ * kp_.ninst;
@@ -2435,9 +2448,9 @@ class Solver : public SolverBase {
   long long staging_n_ = 0;
   FftPlan<A> px_{}, py_{}, pxb_{}, pyb_{};
   // twiddles of the register transforms (null: the length is not one of
-  // theirs): x rows, y columns of ny and 3 ny / 2
+  // theirs): x rows, y columns of ny and 3 ny / 2, 3/2-grid x rows
   bool rf_ = true;
-  T2 *rx_tw_ = nullptr, *ry_twn_ = nullptr, *ry_twm_ = nullptr;
+  T2 *rx_tw_ = nullptr, *ry_twn_ = nullptr, *ry_twm_ = nullptr, *rxb_tw_ = nullptr;
   A *kxw_ = nullptr, *kyw_ = nullptr, *G1_ = nullptr, *G2_ = nullptr;
   int kmax_g_[2] = {1 << 30, 1 << 30};   // largest kx column with a nonzero G1 / G2 weight
   double *kxw64_ = nullptr, *kyw64_ = nullptr;
