@@ -477,395 +477,177 @@ __global__ void k_interp(InterpArgs<R> a) {
 // pressure solve per (kx, ky) column in FP64, the kx = ky = 0 mode by
 // vertical integration, Nyquist rows zeroed.  Spectra layout [level][jy][kx].
 //
-// The pivots of the Thomas elimination depend only on (kx, ky, dz), so
-// ibet_j = 1/bet_j and gam_j are computed once per grid (host, FP64, the
-// reference's recurrence) and a zero pivot is reported when the solver is
-// created.  Each column's sweeps are split into SEG segments worked on by
-// SEG threads: a first pass per segment composes the affine map from the
-// segment's input value to its end value, shared memory chains the maps
-// across segments, and a second pass re-sweeps every segment from its exact
-// input in the reference's order: u_j = (r_j - a_j u_{j-1}) / bet_j forward,
-// u_j = u_j - gam_{j+1} u_{j+1} backward.
+// Each column is eliminated from both ends to the middle and substituted back
+// outwards.  The pivots depend only on (kx, ky, dz) and the matrix is
+// symmetric off its first and last rows, so one factor per unknown (made once
+// per grid on the host) serves both directions of both halves.  With q = 0
+// the end's row, c = 1/dz^2 and r the right-hand side over c:
+//   u_q = g_q (r_q - u_{q-1})                       inwards,
+//   x = i (u + g u') at the middle, u' the other half's u, i = 1 / (1 - g g'),
+//   x_q = u_q - g_q x_{q+1}                         outwards,
+// with g = c / bet in the interior and -1 in the end rows.  The upper half
+// runs on negated values, so that both halves are one code.  The spectra
+// arrive scaled by dz (SrcFields), which leaves
+//   r = i kx dz Hx + i ky dz Hy + Hz(j) - Hz(j-1).
+//
+// Bound by the FP64 pipe (1/64 of the FP32 rate): six FP64 operations per
+// unknown and component; a sweep in segments joined through shared memory
+// needs about four times as many.  One thread has one component (real or
+// imaginary: the matrix is real) of one half of a column, so that a single
+// instance's columns give every SM several warps, whose loads and integer
+// work run under one another's FP64 operations.  Measured, us per launch
+// against the segmented and sequential forms before (and the FP64 operations
+// at the pipe's rate): one 128^3 instance 34.5 (84.6; 26), 256x256x192 171
+// (364; 154), the 48-instance ensemble 61 per class (132; 56), one 48^3
+// instance 14.5 (19.9; latency).  Dropped: one sweep per column and component
+// from one end (44 us at 128^3: half the warps, twice the chain), and FP32
+// spectra widened in the solve (51 us: the integer work then bounds it).
 // ---------------------------------------------------------------------------
-// SEG segments per column, COLS columns per block (SEG * COLS threads).
-// The host picks among this looped form, the register-held k_thomas_r and
-// the sequential k_thomas_seq (below) by column count and unknowns.
-
-struct ThomasArgs {
-  const double2 *Hx, *Hy, *Hz;   // levels 1..nz at index level-1, [inst][nz][P]
-  const double2 *Hb, *Ht;        // r2c of divtz(1), divtz(nz) (scaled), [inst][2][P]
-  double2* phat;                 // levels 0..nz, [inst][nz+1][P]; holds r, then u
-  const double *ibet, *gam;      // [n+1][P], index j = 1..n (shared by instances)
+struct ThomasArgs {   // (real, imaginary) pairs
+  const double *Hx, *Hy, *Hz;   // levels 1..nz at index level-1, [inst][nz][P], dz-scaled
+  const double* Hb;         // r2c of divtz(1), divtz(nz) (scaled), [inst][2][P]
+  double* phat;             // levels 0..nz, [inst][nz+1][P]; holds u, then the result
+  const double* g;          // [n+1][P]: i of the column, then g of unknowns 1..n (shared by instances)
   const double *kxw, *kyw;
-  double dz, idz, idz2;   // dz, 1/dz, 1/dz^2 (made on the host)
+  double dz;
   int nz, ny, K, ninst;
 };
 
-__device__ __forceinline__ double2 thomas_rhs(const ThomasArgs& a, const double2* Hx, const double2* Hy,
-                                              const double2* Hz, const double2* Hb, const double2* Ht, int j,
-                                              long long P, int t, double kxv, double kyv) {
-  const int nz = a.nz;
-  if (j == 1) { const double2 h = Hb[t]; return make_double2(-a.dz * h.x, -a.dz * h.y); }
-  if (j == nz + 1) { const double2 h = Ht[t]; return make_double2(-a.dz * h.x, -a.dz * h.y); }
-  const double c4 = a.idz;
-  const double2 hx = Hx[(j - 2) * P + t], hy = Hy[(j - 2) * P + t];
-  const double2 hz = Hz[(j - 1) * P + t], hzp = Hz[(j - 2) * P + t];
-  // i kx Hx(j-1) + i ky Hy(j-1) + (Hz(j) - Hz(j-1)) / dz
-  return make_double2((-hx.y * kxv) + (-hy.y * kyv) + (hz.x - hzp.x) * c4,
-                      (hx.x * kxv) + (hy.x * kyv) + (hz.y - hzp.y) * c4);
-}
-
-template <int SEG, int COLS>
-__global__ void __launch_bounds__(SEG * COLS) k_thomas(ThomasArgs a) {
-  __shared__ double2 s_x[SEG][COLS];   // segment end value / start value
-  __shared__ double s_h[SEG][COLS];    // segment map slope
-  const int lane = threadIdx.x % COLS, seg = threadIdx.x / COLS;
-  const long long P = (long long)a.ny * a.K;
-  const long long gcol = (long long)blockIdx.x * COLS + lane;
-  const bool live = gcol < P * a.ninst;
-  const int inst = live ? (int)(gcol / P) : 0;
-  const int t = live ? (int)(gcol - inst * P) : 0;
-  const int jy = t / a.K, kx = t - jy * a.K;
+template <int C>
+__global__ void __launch_bounds__(32) k_thomas(ThomasArgs a) {
+  const int P = a.ny * a.K, P2 = 2 * P;
   const int nz = a.nz, n = nz + 1;
-  const double2* Hx = a.Hx + (long long)inst * nz * P;
-  const double2* Hy = a.Hy + (long long)inst * nz * P;
-  const double2* Hz = a.Hz + (long long)inst * nz * P;
-  const double2* Hb = a.Hb + (long long)inst * 2 * P;
-  const double2* Ht = a.Ht + (long long)inst * 2 * P;
-  double2* phat = a.phat + (long long)inst * (nz + 1) * P;   // u_j at phat[(j-1)*P]
-  const bool nyq = jy == a.ny / 2;
-  const bool mean = kx == 0 && jy == 0;
-  const int L = (n + SEG - 1) / SEG;
-  const int j0 = 1 + seg * L, j1 = min(n, j0 + L - 1);   // this thread's levels (may be empty)
-  const double c3 = a.idz2;
-  const double kxv = a.kxw[kx], kyv = a.kyw[jy];
-  const bool solve = live && !nyq && !mean;
-
-  // ---- forward: r_j into phat, and the segment's map x -> u_{j1} = ut + h x
-  double2 ut = make_double2(0.0, 0.0);
-  double h = 1.0;
-  if (solve) {
-    for (int j = j0; j <= j1; ++j) {
-      const double2 r = thomas_rhs(a, Hx, Hy, Hz, Hb, Ht, j, P, t, kxv, kyv);
-      phat[(j - 1) * P + t] = r;
-      const double ib = a.ibet[(long long)j * P + t];
-      const double aj = (j == 1) ? 0.0 : (j <= nz ? c3 : -1.0);
-      ut = make_double2((r.x - aj * ut.x) * ib, (r.y - aj * ut.y) * ib);
-      h = -aj * ib * h;
-    }
-  }
-  s_x[seg][lane] = ut;
-  s_h[seg][lane] = h;
-  __syncthreads();
-  double2 x = make_double2(0.0, 0.0);   // u_{j0-1}
-  for (int s = 0; s < seg; ++s) {
-    const double2 e = s_x[s][lane];
-    const double hs = s_h[s][lane];
-    x = make_double2(e.x + hs * x.x, e.y + hs * x.y);
-  }
-  __syncthreads();
-  // ---- forward re-sweep from the exact input; the segment end is u_{j1}
-  double2 up = x;
-  if (solve) {
-    for (int j = j0; j <= j1; ++j) {
-      const double2 r = phat[(j - 1) * P + t];
-      const double ib = a.ibet[(long long)j * P + t];
-      const double aj = (j == 1) ? 0.0 : (j <= nz ? c3 : -1.0);
-      up = make_double2((r.x - aj * up.x) * ib, (r.y - aj * up.y) * ib);
-      phat[(j - 1) * P + t] = up;
-    }
-  }
-  // ---- backward: v_j = u_j - gam_{j+1} v_{j+1}; map y = v_{j1+1} -> v_{j0} = vt + g y
-  double2 vt = make_double2(0.0, 0.0);
-  double g = 1.0;
-  if (solve) {
-    for (int j = j1; j >= j0; --j) {
-      const double2 uj = phat[(j - 1) * P + t];
-      const double gj = (j == n) ? 0.0 : a.gam[(long long)(j + 1) * P + t];
-      vt = make_double2(uj.x - gj * vt.x, uj.y - gj * vt.y);
-      g = -gj * g;
-    }
-  }
-  s_x[seg][lane] = vt;
-  s_h[seg][lane] = g;
-  __syncthreads();
-  double2 y = make_double2(0.0, 0.0);   // v_{j1+1}; the top segment has none
-  for (int s = SEG - 1; s > seg; --s) {
-    const double2 e = s_x[s][lane];
-    const double gs = s_h[s][lane];
-    y = make_double2(e.x + gs * y.x, e.y + gs * y.y);
-  }
-  if (solve) {
-    double2 vn = y;
-    for (int j = j1; j >= j0; --j) {
-      double2 uj = phat[(j - 1) * P + t];
-      if (j < n) {
-        const double gj = a.gam[(long long)(j + 1) * P + t];
-        uj = make_double2(uj.x - gj * vn.x, uj.y - gj * vn.y);
-      }
-      phat[(j - 1) * P + t] = uj;
-      vn = uj;
-    }
-  }
-  if (!live) return;
-  if (nyq) {
-    for (int j = j0; j <= j1; ++j) phat[(j - 1) * P + t] = make_double2(0.0, 0.0);
-  } else if (mean && seg == 0) {
-    // kx = ky = 0: p(0) = 0, p(1) = -dz rbottomw, p(jz) = p(jz-1) + Hz(jz) dz
-    double2 p = make_double2(0.0, 0.0);
-    phat[t] = p;
-    const double2 hb = Hb[t];
-    p = make_double2(p.x - a.dz * hb.x, p.y - a.dz * hb.y);
-    phat[P + t] = p;
-    for (int jz = 2; jz <= nz; ++jz) {
-      const double2 hz = Hz[(jz - 1) * P + t];
-      p = make_double2(p.x + hz.x * a.dz, p.y + hz.y * a.dz);
-      phat[jz * P + t] = p;
-    }
-  }
-}
-
-// The same solve with each thread's segment (at most LMAX levels) held in
-// registers: all of the segment's loads (right-hand side inputs, pivots)
-// are issued before the recurrences run, and phat is written once.  The
-// arithmetic is k_thomas's, operation for operation.
-template <int SEG, int COLS, int LMAX>
-__global__ void __launch_bounds__(SEG * COLS) k_thomas_r(ThomasArgs a) {
-  __shared__ double2 s_x[SEG][COLS];
-  __shared__ double s_h[SEG][COLS];
-  const int lane = threadIdx.x % COLS, seg = threadIdx.x / COLS;
-  const long long P = (long long)a.ny * a.K;
-  const long long gcol = (long long)blockIdx.x * COLS + lane;
-  const bool live = gcol < P * a.ninst;
-  const int inst = live ? (int)(gcol / P) : 0;
-  const int t = live ? (int)(gcol - inst * P) : 0;
-  const int jy = t / a.K, kx = t - jy * a.K;
-  const int nz = a.nz, n = nz + 1;
-  const double2* Hx = a.Hx + (long long)inst * nz * P;
-  const double2* Hy = a.Hy + (long long)inst * nz * P;
-  const double2* Hz = a.Hz + (long long)inst * nz * P;
-  const double2* Hb = a.Hb + (long long)inst * 2 * P;
-  const double2* Ht = a.Ht + (long long)inst * 2 * P;
-  double2* phat = a.phat + (long long)inst * (nz + 1) * P;
-  const bool nyq = jy == a.ny / 2;
-  const bool mean = kx == 0 && jy == 0;
-  const int L = (n + SEG - 1) / SEG;
-  const int j0 = 1 + seg * L, j1 = min(n, j0 + L - 1);
-  const double c3 = a.idz2;
-  const double kxv = a.kxw[kx], kyv = a.kyw[jy];
-  const bool solve = live && !nyq && !mean;
-  double2 rr[LMAX];
-  double ib[LMAX], gm[LMAX];
+  const int nmean = 2 * a.ninst;   // the first blocks: the mean modes
+  if ((int)blockIdx.x < nmean) {
+    // kx = ky = 0: p(0) = 0, p(1) = -dz rbottomw, p(jz) = p(jz-1) + Hz(jz) dz,
+    // a run of levels per lane, the runs joined by a scan of their sums
+    const int inst = blockIdx.x >> 1, comp = blockIdx.x & 1, lane = threadIdx.x;
+    const double* Hz = a.Hz + (long long)inst * nz * P2 + comp;
+    double* out = a.phat + (long long)inst * n * P2 + comp;
+    const int run = (nz + 30) / 32, k0 = 2 + lane * run, k1 = min(k0 + run, nz + 1);
+    double own = 0.0;
+#pragma unroll 8
+    for (int k = k0; k < k1; ++k) own += Hz[(long long)(k - 1) * P2];
+    double sum = own;
 #pragma unroll
-  for (int m = 0; m < LMAX; ++m) {
-    const int j = j0 + m;
-    rr[m] = make_double2(0.0, 0.0);
-    ib[m] = 0.0;
-    gm[m] = 0.0;
-    if (solve && j <= j1) {
-      rr[m] = thomas_rhs(a, Hx, Hy, Hz, Hb, Ht, j, P, t, kxv, kyv);
-      ib[m] = a.ibet[(long long)j * P + t];
-      if (j < n) gm[m] = a.gam[(long long)(j + 1) * P + t];
+    for (int d = 1; d < 32; d *= 2) {
+      const double o = __shfl_up_sync(0xffffffffu, sum, d);
+      if (lane >= d) sum += o;
     }
-  }
-  // forward map x -> u_{j1} = ut + h x
-  double2 ut = make_double2(0.0, 0.0);
-  double h = 1.0;
-#pragma unroll
-  for (int m = 0; m < LMAX; ++m) {
-    const int j = j0 + m;
-    if (solve && j <= j1) {
-      const double aj = (j == 1) ? 0.0 : (j <= nz ? c3 : -1.0);
-      ut = make_double2((rr[m].x - aj * ut.x) * ib[m], (rr[m].y - aj * ut.y) * ib[m]);
-      h = -aj * ib[m] * h;
+    const double p1 = -(a.dz * a.Hb[(long long)inst * 2 * P2 + comp]);
+    if (lane == 0) {
+      out[0] = 0.0;
+      out[P2] = p1;
     }
-  }
-  s_x[seg][lane] = ut;
-  s_h[seg][lane] = h;
-  __syncthreads();
-  double2 x = make_double2(0.0, 0.0);
-  for (int s = 0; s < seg; ++s) {
-    const double2 e = s_x[s][lane];
-    const double hs = s_h[s][lane];
-    x = make_double2(e.x + hs * x.x, e.y + hs * x.y);
-  }
-  __syncthreads();
-  // forward re-sweep from the exact input: rr becomes u
-  double2 up = x;
-#pragma unroll
-  for (int m = 0; m < LMAX; ++m) {
-    const int j = j0 + m;
-    if (solve && j <= j1) {
-      const double aj = (j == 1) ? 0.0 : (j <= nz ? c3 : -1.0);
-      up = make_double2((rr[m].x - aj * up.x) * ib[m], (rr[m].y - aj * up.y) * ib[m]);
-      rr[m] = up;
-    }
-  }
-  // backward map y = v_{j1+1} -> v_{j0} = vt + g y
-  double2 vt = make_double2(0.0, 0.0);
-  double g = 1.0;
-#pragma unroll
-  for (int m = LMAX - 1; m >= 0; --m) {
-    const int j = j0 + m;
-    if (solve && j <= j1) {
-      const double gj = gm[m];   // 0 at j = n
-      vt = make_double2(rr[m].x - gj * vt.x, rr[m].y - gj * vt.y);
-      g = -gj * g;
-    }
-  }
-  s_x[seg][lane] = vt;
-  s_h[seg][lane] = g;
-  __syncthreads();
-  double2 y = make_double2(0.0, 0.0);
-  for (int s = SEG - 1; s > seg; --s) {
-    const double2 e = s_x[s][lane];
-    const double gs = s_h[s][lane];
-    y = make_double2(e.x + gs * y.x, e.y + gs * y.y);
-  }
-  if (solve) {
-    double2 vn = y;
-#pragma unroll
-    for (int m = LMAX - 1; m >= 0; --m) {
-      const int j = j0 + m;
-      if (j <= j1) {
-        double2 uj = rr[m];
-        if (j < n) uj = make_double2(uj.x - gm[m] * vn.x, uj.y - gm[m] * vn.y);
-        phat[(j - 1) * P + t] = uj;
-        vn = uj;
-      }
-    }
-  }
-  if (!live) return;
-  if (nyq) {
-    for (int j = j0; j <= j1; ++j) phat[(j - 1) * P + t] = make_double2(0.0, 0.0);
-  } else if (mean && seg == 0) {
-    double2 p = make_double2(0.0, 0.0);
-    phat[t] = p;
-    const double2 hb = Hb[t];
-    p = make_double2(p.x - a.dz * hb.x, p.y - a.dz * hb.y);
-    phat[P + t] = p;
-    for (int jz = 2; jz <= nz; ++jz) {
-      const double2 hz = Hz[(jz - 1) * P + t];
-      p = make_double2(p.x + hz.x * a.dz, p.y + hz.y * a.dz);
-      phat[jz * P + t] = p;
-    }
-  }
-}
-
-// The sequential form: one thread per column sweeps all n levels in the
-// reference's order (forward u_j = (r_j - a_j u_{j-1}) / bet_j, then
-// u_j -= gam_{j+1} u_{j+1}), with half the FP64 work of the segmented form
-// (no segment maps).  Chunks of C levels are double-buffered in registers:
-// the next chunk's loads are in flight while the current one is swept.
-template <int C>
-__device__ __forceinline__ void thomas_fwd_load(const ThomasArgs& a, const double2* Hx, const double2* Hy,
-                                                const double2* Hz, const double2* Hb, const double2* Ht,
-                                                long long P, int t, double kxv, double kyv, int j0, int n,
-                                                double2* rr, double* ib) {
-#pragma unroll
-  for (int m = 0; m < C; ++m) {
-    const int j = j0 + m;
-    if (j <= n) {
-      rr[m] = thomas_rhs(a, Hx, Hy, Hz, Hb, Ht, j, P, t, kxv, kyv);
-      ib[m] = a.ibet[(long long)j * P + t];
-    }
-  }
-}
-
-template <int C>
-__device__ __forceinline__ void thomas_fwd_sweep(double2* phat, long long P, int t, int j0, int n, int nz,
-                                                 double c3, const double2* rr, const double* ib, double2& up) {
-#pragma unroll
-  for (int m = 0; m < C; ++m) {
-    const int j = j0 + m;
-    if (j <= n) {
-      const double aj = (j == 1) ? 0.0 : (j <= nz ? c3 : -1.0);
-      up = make_double2((rr[m].x - aj * up.x) * ib[m], (rr[m].y - aj * up.y) * ib[m]);
-      phat[(j - 1) * P + t] = up;
-    }
-  }
-}
-
-template <int C>
-__device__ __forceinline__ void thomas_bwd_load(const ThomasArgs& a, const double2* phat, long long P, int t, int j1,
-                                                double2* uu, double* gg) {
-#pragma unroll
-  for (int m = 0; m < C; ++m) {
-    const int j = j1 - m;
-    if (j >= 1) {
-      uu[m] = phat[(j - 1) * P + t];
-      gg[m] = a.gam[(long long)(j + 1) * P + t];
-    }
-  }
-}
-
-template <int C>
-__device__ __forceinline__ void thomas_bwd_sweep(double2* phat, long long P, int t, int j1, const double2* uu,
-                                                 const double* gg, double2& vn) {
-#pragma unroll
-  for (int m = 0; m < C; ++m) {
-    const int j = j1 - m;
-    if (j >= 1) {
-      vn = make_double2(uu[m].x - gg[m] * vn.x, uu[m].y - gg[m] * vn.y);
-      phat[(j - 1) * P + t] = vn;
-    }
-  }
-}
-
-template <int C>
-__global__ void __launch_bounds__(128) k_thomas_seq(ThomasArgs a) {
-  const long long P = (long long)a.ny * a.K;
-  const long long gcol = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (gcol >= P * a.ninst) return;
-  const int inst = (int)(gcol / P);
-  const int t = (int)(gcol - inst * P);
-  const int jy = t / a.K, kx = t - jy * a.K;
-  const int nz = a.nz, n = nz + 1;
-  const double2* Hx = a.Hx + (long long)inst * nz * P;
-  const double2* Hy = a.Hy + (long long)inst * nz * P;
-  const double2* Hz = a.Hz + (long long)inst * nz * P;
-  const double2* Hb = a.Hb + (long long)inst * 2 * P;
-  const double2* Ht = a.Ht + (long long)inst * 2 * P;
-  double2* phat = a.phat + (long long)inst * (nz + 1) * P;
-  if (jy == a.ny / 2) {
-    for (int j = 1; j <= n; ++j) phat[(j - 1) * P + t] = make_double2(0.0, 0.0);
-    return;
-  }
-  if (kx == 0 && jy == 0) {
-    double2 p = make_double2(0.0, 0.0);
-    phat[t] = p;
-    const double2 hb = Hb[t];
-    p = make_double2(p.x - a.dz * hb.x, p.y - a.dz * hb.y);
-    phat[P + t] = p;
-    for (int jz = 2; jz <= nz; ++jz) {
-      const double2 hz = Hz[(jz - 1) * P + t];
-      p = make_double2(p.x + hz.x * a.dz, p.y + hz.y * a.dz);
-      phat[jz * P + t] = p;
+    double p = p1 + (sum - own);
+#pragma unroll 8
+    for (int k = k0; k < k1; ++k) {
+      p += Hz[(long long)(k - 1) * P2];
+      out[(long long)k * P2] = p;
     }
     return;
   }
-  const double c3 = a.idz2;
-  const double kxv = a.kxw[kx], kyv = a.kyw[jy];
-  double2 rA[C], rB[C];
-  double iA[C], iB[C];
-  double2 up = make_double2(0.0, 0.0);
-  thomas_fwd_load<C>(a, Hx, Hy, Hz, Hb, Ht, P, t, kxv, kyv, 1, n, rA, iA);
-  for (int j0 = 1; j0 <= n; j0 += 2 * C) {
-    thomas_fwd_load<C>(a, Hx, Hy, Hz, Hb, Ht, P, t, kxv, kyv, j0 + C, n, rB, iB);
-    thomas_fwd_sweep<C>(phat, P, t, j0, n, nz, c3, rA, iA, up);
-    thomas_fwd_load<C>(a, Hx, Hy, Hz, Hb, Ht, P, t, kxv, kyv, j0 + 2 * C, n, rA, iA);
-    thomas_fwd_sweep<C>(phat, P, t, j0 + C, n, nz, c3, rB, iB, up);
+  const int half = threadIdx.x >> 4, comp = threadIdx.x & 1;   // eight columns per warp
+  const long long gcol = (long long)(blockIdx.x - nmean) * 8 + ((threadIdx.x & 15) >> 1);
+  const bool live = gcol < (long long)P * a.ninst;
+  const int inst = live ? (int)(gcol / P) : 0, t = live ? (int)(gcol - (long long)inst * P) : 1;
+  const int jy = t / a.K, kx = t - jy * a.K;
+  const int e = 2 * t + comp, eo = 2 * t + 1 - comp;
+  const bool nyq = jy == a.ny / 2, store = live && t != 0;
+  // this half's unknowns q = 0 .. cnt, in steps of sd levels from the end
+  const int m = n / 2, cnt = half ? n - 1 - m : m - 1, most = n - 1 - m;
+  const int sd = half ? -P2 : P2, sg = half ? -P : P;
+  double* out = a.phat + (long long)inst * n * P2 + (half ? (long long)(n - 1) * P2 : 0) + e;
+  // row q >= 1: Hx, Hy at x + (q-1) sd, the new Hz at z + q sd
+  const double* x = a.Hx + ((long long)inst * nz + (half ? nz - 2 : 0)) * P2 + eo;
+  const double* y = a.Hy + ((long long)inst * nz + (half ? nz - 2 : 0)) * P2 + eo;
+  const double* z = a.Hz + ((long long)inst * nz + (half ? nz - 1 : 0)) * P2 + e;
+  const double* g = a.g + (long long)(half ? n : 1) * P + t;
+  const bool neg = (comp == 0) != (half == 1);
+  const double kxs = (neg ? -a.kxw[kx] : a.kxw[kx]) * a.dz, kys = (neg ? -a.kyw[jy] : a.kyw[jy]) * a.dz;
+
+  struct Chunk { double x[C], y[C], z[C], g[C]; };
+  auto load = [&](int q0, Chunk& c) {   // rows q0 .. q0 + C - 1, up to cnt
+#pragma unroll
+    for (int i = 0; i < C; ++i) {
+      const int q = min(q0 + i, cnt), o = q * sd;
+      c.x[i] = x[o - sd];
+      c.y[i] = y[o - sd];
+      c.z[i] = z[o];
+      c.g[i] = g[q * sg];
+    }
+  };
+  double up = a.dz * a.Hb[((long long)inst * 2 + half) * P2 + e], zp = z[0];
+  if (store) out[0] = up;
+  // a chunk's right-hand sides first: they are independent, and the FP64
+  // latency then falls on the recurrence's one operation per row alone
+  auto sweep = [&](int q0, const Chunk& c, bool full) {
+    double r[C];
+#pragma unroll
+    for (int i = 0; i < C; ++i)
+      r[i] = fma(kxs, c.x[i], fma(kys, c.y[i], c.z[i] - (i ? c.z[i - 1] : zp)));
+    zp = c.z[C - 1];
+#pragma unroll
+    for (int i = 0; i < C; ++i) r[i] = c.g[i] * r[i];
+    if (full) {
+#pragma unroll
+      for (int i = 0; i < C; ++i) {
+        up = fma(-c.g[i], up, r[i]);
+        if (store) out[(q0 + i) * sd] = up;
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < C; ++i)
+        if (q0 + i <= cnt) {
+          up = fma(-c.g[i], up, r[i]);
+          if (store) out[(q0 + i) * sd] = up;
+        }
+    }
+  };
+  {
+    Chunk c[4];   // three chunks in flight under the sweep of the fourth
+#pragma unroll
+    for (int s = 0; s < 3; ++s) load(1 + s * C, c[s]);
+    for (int q0 = 1; q0 <= most; q0 += 4 * C) {
+      const bool full = q0 + 4 * C - 1 < most;   // the lower half may have one row fewer
+#pragma unroll
+      for (int s = 0; s < 4; ++s) {
+        load(q0 + (s + 3) * C, c[(s + 3) & 3]);
+        sweep(q0 + s * C, c[s], full);
+      }
+    }
   }
-  // u_n stays; levels n-1 .. 1
-  double2 vn = up;
-  double2 uA[C], uB[C];
-  double gA[C], gB[C];
-  thomas_bwd_load<C>(a, phat, P, t, n - 1, uA, gA);
-  for (int j1 = n - 1; j1 >= 1; j1 -= 2 * C) {
-    thomas_bwd_load<C>(a, phat, P, t, j1 - C, uB, gB);
-    thomas_bwd_sweep<C>(phat, P, t, j1, uA, gA, vn);
-    thomas_bwd_load<C>(a, phat, P, t, j1 - 2 * C, uA, gA);
-    thomas_bwd_sweep<C>(phat, P, t, j1 - C, uB, gB, vn);
+  // the middle, then outwards: unknowns cnt .. 0
+  const unsigned flip = half ? 0x80000000u : 0u;
+  up = a.g[t] * fma(g[cnt * sg], __shfl_xor_sync(0xffffffffu, up, 16), up);
+  if (nyq) up = 0.0;
+  if (store) out[cnt * sd] = half ? -up : up;
+  struct Back { double u[C], g[C]; };
+  auto bload = [&](int q0, Back& c) {   // unknowns q0, q0 - 1, .., down to 0
+#pragma unroll
+    for (int i = 0; i < C; ++i) {
+      const int q = max(q0 - i, 0);
+      c.u[i] = out[q * sd];
+      c.g[i] = g[q * sg];
+    }
+  };
+  auto bsweep = [&](int q0, const Back& c) {
+#pragma unroll
+    for (int i = 0; i < C; ++i) {
+      up = fma(-c.g[i], up, c.u[i]);
+      if (q0 - i >= 0 && store)   // the upper half's sign: an integer operation
+        out[(q0 - i) * sd] = nyq ? 0.0 : __hiloint2double((int)((unsigned)__double2hiint(up) ^ flip), __double2loint(up));
+    }
+  };
+  Back c[4];
+#pragma unroll
+  for (int s = 0; s < 3; ++s) bload(cnt - 1 - s * C, c[s]);
+  for (int q0 = cnt - 1; q0 >= 0; q0 -= 4 * C) {
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      bload(q0 - (s + 3) * C, c[(s + 3) & 3]);
+      bsweep(q0 - s * C, c[s]);
+    }
   }
 }
 

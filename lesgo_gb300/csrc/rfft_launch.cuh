@@ -68,7 +68,7 @@ void ry_spec(const RyArgs<A, cplx<A>, double2>& a, int ny, int nlev, int nf, cud
   with_ry(ny, [&](auto len) {
     constexpr int R1 = decltype(len)::R1, R2 = decltype(len)::R2;
     constexpr size_t smem = ry_elems<R1, R2>() * sizeof(cplx<A>);
-    auto kern = k_ry_spec<A, double2, R1, R2>;
+    auto kern = k_ry_spec<A, R1, R2>;
     smem_for(kern, smem);
     kern<<<dim3((a.K + kYC - 1) / kYC, nlev, nf), kYC * cmax(R1, R2), smem, st>>>(a);
   });
@@ -83,8 +83,8 @@ void ry_phys(bool grad, const RyArgs<A, double2, cplx<A>>& a, int ny, int nlev, 
       smem_for(kern, smem);
       kern<<<grid, kYC * cmax(R1, R2), smem, st>>>(a);
     };
-    if (grad) go(k_ry_phys<A, double2, R1, R2, true>, 2 * e);
-    else go(k_ry_phys<A, double2, R1, R2, false>, e);
+    if (grad) go(k_ry_phys<A, R1, R2, true>, 2 * e);
+    else go(k_ry_phys<A, R1, R2, false>, e);
   });
 }
 

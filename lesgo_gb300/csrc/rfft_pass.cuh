@@ -102,7 +102,7 @@ template <int CNT, int STEP, typename R, int NF>
 __device__ __forceinline__ void rx_load(const SrcFields<R, NF>& s, int f, int jy, int li, int n0, cplx<R>* v) {
   const int inst = s.im.inst(li), lv = li - inst * s.im.nli;
   const R* p = pick(s.p, f) + inst * s.im.istr + (long long)(s.lev0 + lv * s.levstride) * s.plane + (long long)jy * s.ld + 2 * n0;
-  const R c = s.isc ? (R)s.isc[inst * SC_N + s.isc_idx] * s.scale : s.scale;   // scale: with the split's 1/2
+  const R c = s.isc ? (R)(s.isc_mul * s.isc[inst * SC_N + s.isc_idx]) : s.scale;
 #pragma unroll
   for (int j = 0; j < CNT; ++j) v[j] = *reinterpret_cast<const cplx<R>*>(p + 2 * STEP * j);
 #pragma unroll
@@ -548,16 +548,44 @@ __device__ __forceinline__ void ry_inv(T2* v, T2* W, const T2* tw, int t, int c)
 }
 template <int R1, int R2> __host__ __device__ constexpr int ry_elems() { return R1 * odd_up(R2) * kYC; }
 
-template <int CNT, typename T2, typename InT>
-__device__ __forceinline__ void ry_load(const InT* p, int step, bool live, T2* v) {
+template <int CNT, typename T2>
+__device__ __forceinline__ void ry_load(const T2* p, int step, bool live, T2* v) {
 #pragma unroll
-  for (int j = 0; j < CNT; ++j) v[j] = live ? cvt2<T2>(p[j * step]) : czero<T2>();
+  for (int j = 0; j < CNT; ++j) v[j] = live ? p[j * step] : czero<T2>();
 }
-template <int CNT, typename T2, typename OutT>
-__device__ __forceinline__ void ry_store(OutT* p, int step, bool live, const T2* v) {
+template <int CNT, typename T2>
+__device__ __forceinline__ void ry_store(T2* p, int step, bool live, const T2* v) {
   if (!live) return;
 #pragma unroll
-  for (int j = 0; j < CNT; ++j) p[j * step] = cvt2<OutT>(v[j]);
+  for (int j = 0; j < CNT; ++j) p[j * step] = v[j];
+}
+// the pressure's FP64 spectra to and from FP32 transforms
+template <int CNT>
+__device__ __forceinline__ void ry_load(const double2* p, int step, bool live, float2* v) {
+  double2 d[CNT];
+  bool odd = false;
+#pragma unroll
+  for (int j = 0; j < CNT; ++j) d[j] = live ? p[j * step] : make_double2(1.0, 1.0);
+#pragma unroll
+  for (int j = 0; j < CNT; ++j) v[j] = make_float2(narrow_fast(d[j].x, odd), narrow_fast(d[j].y, odd));
+  if (odd) {
+#pragma unroll
+    for (int j = 0; j < CNT; ++j) v[j] = make_float2((float)d[j].x, (float)d[j].y);
+  }
+}
+template <int CNT>
+__device__ __forceinline__ void ry_store(double2* p, int step, bool live, const float2* v) {
+  if (!live) return;
+  double2 d[CNT];
+  bool odd = false;
+#pragma unroll
+  for (int j = 0; j < CNT; ++j) d[j] = make_double2(widen_fast(v[j].x, odd), widen_fast(v[j].y, odd));
+  if (odd) {
+#pragma unroll
+    for (int j = 0; j < CNT; ++j) d[j] = make_double2((double)v[j].x, (double)v[j].y);
+  }
+#pragma unroll
+  for (int j = 0; j < CNT; ++j) p[j * step] = d[j];
 }
 // v[k2] *= i ky of row t + R1 k2 (zero in the Nyquist row of the table)
 template <typename A, int R1, int R2>
@@ -592,7 +620,7 @@ __global__ void __launch_bounds__(kYC * cmax(R1, R2)) k_ry_filt(RyArgs<A, cplx<A
   T2* ny = W1 + E;
   const T2* src = a.in + f * a.in_fs + pin * N * a.K + t * a.K + kx;
   T2 v[cmax(R1, R2)];
-  if (t < R2) ry_load<R1, T2>(src, R2 * a.K, live, v);
+  if (t < R2) ry_load<R1>(src, R2 * a.K, live, v);
   ry_fwd<T2, R1, R2>(v, W0, a.twn, t, c);
   if (t == 0) ny[c] = v[R2 / 2];
   ry_iky<A, R1, R2>(a.kyw, t, v);
@@ -602,7 +630,7 @@ __global__ void __launch_bounds__(kYC * cmax(R1, R2)) k_ry_filt(RyArgs<A, cplx<A
     ry_store<R1>(d + 2 * a.out_fs, R2 * a.K, true, v);
     const T2 s = (t & 1) ? mkc(-ny[c].x, -ny[c].y) : ny[c];
     const A k = a.kxw[kx], n = (A)N;
-    ry_load<R1, T2>(src, R2 * a.K, true, v);
+    ry_load<R1>(src, R2 * a.K, true, v);
 #pragma unroll
     for (int j = 0; j < R1; ++j) {
       const T2 x = csub(cscale(v[j], n), s);
@@ -625,12 +653,12 @@ __global__ void __launch_bounds__(kYC * cmax(R1, R2)) k_ry_div(RyArgs<A, cplx<A>
   const T2* qq = a.in + pick(a.ib, f) * a.in_fs + pin * N * a.K + t * a.K + kx;
   T2 v[cmax(R1, R2)];
   if (t < R2) {
-    ry_load<R1, T2>(pp, R2 * a.K, live, v);
+    ry_load<R1>(pp, R2 * a.K, live, v);
     T2 s = v[0];
 #pragma unroll
     for (int j = 1; j < R1; ++j) s = cadd(s, v[j]);
     sum[t * kYC + c] = (t & 1) ? mkc(-s.x, -s.y) : s;
-    ry_load<R1, T2>(qq, R2 * a.K, live, v);
+    ry_load<R1>(qq, R2 * a.K, live, v);
   }
   ry_fwd<T2, R1, R2>(v, W0, a.twn, t, c);
   ry_iky<A, R1, R2>(a.kyw, t, v);
@@ -643,7 +671,7 @@ __global__ void __launch_bounds__(kYC * cmax(R1, R2)) k_ry_div(RyArgs<A, cplx<A>
     const A k = a.kxw[kx], n = (A)N;
     T2* d = a.out + f * a.out_fs + (long long)li * N * a.K + t * a.K + kx;
     T2 x[R1];
-    ry_load<R1, T2>(pp, R2 * a.K, true, x);
+    ry_load<R1>(pp, R2 * a.K, true, x);
 #pragma unroll
     for (int j = 0; j < R1; ++j) {
       const T2 y = csub(cscale(x[j], n), s);
@@ -659,7 +687,7 @@ __global__ void __launch_bounds__(kYC * cmax(R1, 3 * R2 / 2)) k_ry_pad(RyArgs<A,
   constexpr int N = R1 * R2, S2 = 3 * R2 / 2, M = R1 * S2;
   T2* W1 = W0 + ry_elems<R1, R2>();
   T2 v[cmax(R1, S2)];
-  if (t < R2) ry_load<R1, T2>(a.in + f * a.in_fs + pin * N * a.K + t * a.K + kx, R2 * a.K, live, v);
+  if (t < R2) ry_load<R1>(a.in + f * a.in_fs + pin * N * a.K + t * a.K + kx, R2 * a.K, live, v);
   ry_fwd<T2, R1, R2>(v, W0, a.twn, t, c);
   if (t < R1) {
 #pragma unroll
@@ -679,7 +707,7 @@ __global__ void __launch_bounds__(kYC * cmax(R1, 3 * R2 / 2)) k_ry_unpad(RyArgs<
   constexpr int N = R1 * R2, S2 = 3 * R2 / 2, M = R1 * S2;
   T2* W1 = W0 + ry_elems<R1, S2>();
   T2 v[cmax(R1, S2)];
-  if (t < S2) ry_load<R1, T2>(a.in + f * a.in_fs + pin * M * a.K + t * a.K + kx, S2 * a.K, live, v);
+  if (t < S2) ry_load<R1>(a.in + f * a.in_fs + pin * M * a.K + t * a.K + kx, S2 * a.K, live, v);
   ry_fwd<T2, R1, S2>(v, W0, a.twm, t, c);
   if (t < R1) {
 #pragma unroll
@@ -690,13 +718,13 @@ __global__ void __launch_bounds__(kYC * cmax(R1, 3 * R2 / 2)) k_ry_unpad(RyArgs<
   if (t < R2) ry_store<R1>(a.out + f * a.out_fs + (long long)li * N * a.K + t * a.K + kx, R2 * a.K, live, v);
 }
 
-// Forward only (the pressure's right-hand sides).
-template <typename A, typename OutT, int R1, int R2>
-__global__ void __launch_bounds__(kYC * cmax(R1, R2)) k_ry_spec(RyArgs<A, cplx<A>, OutT> a) {
+// Forward only, to FP64 spectra (the pressure's right-hand sides).
+template <typename A, int R1, int R2>
+__global__ void __launch_bounds__(kYC * cmax(R1, R2)) k_ry_spec(RyArgs<A, cplx<A>, double2> a) {
   LESGO_RY_HEAD();
   constexpr int N = R1 * R2;
   T2 v[cmax(R1, R2)];
-  if (t < R2) ry_load<R1, T2>(a.in + f * a.in_fs + pin * N * a.K + t * a.K + kx, R2 * a.K, live, v);
+  if (t < R2) ry_load<R1>(a.in + f * a.in_fs + pin * N * a.K + t * a.K + kx, R2 * a.K, live, v);
   ry_fwd<T2, R1, R2>(v, W0, a.twn, t, c);
   if (t < R1) {
     if (t == 0) v[R2 / 2] = czero<T2>();
@@ -705,15 +733,15 @@ __global__ void __launch_bounds__(kYC * cmax(R1, R2)) k_ry_spec(RyArgs<A, cplx<A
 }
 
 // Inverse only: P -> p (GRAD: and i kx p, i ky p).
-template <typename A, typename InT, int R1, int R2, bool GRAD>
-__global__ void __launch_bounds__(kYC * cmax(R1, R2)) k_ry_phys(RyArgs<A, InT, cplx<A>> a) {
+template <typename A, int R1, int R2, bool GRAD>
+__global__ void __launch_bounds__(kYC * cmax(R1, R2)) k_ry_phys(RyArgs<A, double2, cplx<A>> a) {
   LESGO_RY_HEAD();
   constexpr int N = R1 * R2;
-  const InT* src = a.in + f * a.in_fs + pin * N * a.K + t * a.K + kx;
+  const double2* src = a.in + f * a.in_fs + pin * N * a.K + t * a.K + kx;
   T2* d = a.out + f * a.out_fs + (long long)li * N * a.K + t * a.K + kx;
   T2 v[cmax(R1, R2)];
   if (t < R1) {
-    ry_load<R2, T2>(src, R1 * a.K, live, v);
+    ry_load<R2>(src, R1 * a.K, live, v);
     if (t == 0) v[R2 / 2] = czero<T2>();
   }
   ry_inv<T2, R1, R2>(v, W0, a.twn, t, c);
@@ -726,7 +754,7 @@ __global__ void __launch_bounds__(kYC * cmax(R1, R2)) k_ry_phys(RyArgs<A, InT, c
     }
   }
   if constexpr (GRAD) {
-    if (t < R1) ry_load<R2, T2>(src, R1 * a.K, live, v);
+    if (t < R1) ry_load<R2>(src, R1 * a.K, live, v);
     ry_iky<A, R1, R2>(a.kyw, t, v);
     ry_inv<T2, R1, R2>(v, W0 + ry_elems<R1, R2>(), a.twn, t, c);
     if (t < R2) ry_store<R1>(d + 2 * a.out_fs, R2 * a.K, live, v);
@@ -753,7 +781,7 @@ __global__ void __launch_bounds__(kYC * cmax(R1, R2)) k_ry_test(RyArgs<A, cplx<A
     }
     return;
   }
-  if (t < R2) ry_load<R1, T2>(a.in + f * a.in_fs + pin * N * a.K + t * a.K + kx, R2 * a.K, live, v);
+  if (t < R2) ry_load<R1>(a.in + f * a.in_fs + pin * N * a.K + t * a.K + kx, R2 * a.K, live, v);
   ry_fwd<T2, R1, R2>(v, W0, a.twn, t, c);
   T2 x[R2];
   auto times = [&](const A* G) {

@@ -203,7 +203,7 @@ static long long footprint_bytes(const Derived& d, int cap) {
   b += (std::max({21 * vs, 6 * vs, 3 * vb}) + std::max({42 * vs, 6 * vb, 9 * vs}) + 4 * ps) * 2 * rs;   // spectra
   b += (std::max(6 * vs, 3 * vb) + std::max(6 * vb, 3 * vs)) * 2 * rs;                             // convec spectra
   b += (3 * vs + 2 * ps + (long long)(d.nz + 1) * ps) * 16;                                          // FP64 pressure
-  return b * cap + 2LL * (d.nz + 2) * ps * 8;                                                       // Thomas pivots
+  return b * cap + (long long)(d.nz + 2) * ps * 8;                                                   // Thomas factors
 }
 
 // Host rounding of a table value to the transforms' arithmetic type (the
@@ -312,8 +312,6 @@ class Solver : public SolverBase {
     if (const char* e = std::getenv("LESGO_YBUDGET")) ybudget_ = (size_t)std::max(8192, std::atoi(e));
     if (const char* e = std::getenv("LESGO_YTHREADS")) ythreads_ = std::atoi(e) == 128 ? 128 : 256;
     if (const char* e = std::getenv("LESGO_YSHORTCUT")) yshort_ = std::strcmp(e, "0") != 0;
-    if (const char* e = std::getenv("LESGO_THOMAS"))
-      thomas_mode_ = std::strcmp(e, "seq") == 0 ? 1 : std::strcmp(e, "seg") == 0 ? 2 : 0;
     // LESGO_RFFT=0: every pass on the run-time radix stages of fft_core.cuh
     if (const char* e = std::getenv("LESGO_RFFT")) rf_ = std::strcmp(e, "0") != 0;
     use_graphs_ = graphs_allowed_;
@@ -1630,12 +1628,12 @@ class Solver : public SolverBase {
     return upload_vec(t);
   }
 
-  // Thomas pivots of every (kx, ky) column (tridag_array.f90:166-246): they
-  // depend only on the wavenumbers and dz, so they are formed once in FP64.
+  // The factors g of k_thomas for every (kx, ky) column, from the pivots of
+  // tridag_array.f90:166-246: they depend only on the wavenumbers and dz.
   void build_thomas_pivots() {
     const int ny = d_.ny, K = d_.K, nz = d_.nz, n = nz + 1;
     const long long P = (long long)ny * K;
-    std::vector<double> ib((size_t)(n + 1) * P, 1.0), gm((size_t)(n + 1) * P, 0.0);
+    std::vector<double> gm((size_t)(n + 1) * P, 0.0);
     const double c3 = 1.0 / (d_.dz * d_.dz);
     for (int jy = 0; jy < ny; ++jy) {
       if (jy == ny / 2) continue;
@@ -1648,21 +1646,25 @@ class Solver : public SolverBase {
         volatile double k2 = kxv * kxv;
         k2 = k2 + kyv * kyv;
         const double bmid = -(k2 + 2.0 * c3);
-        double bet = -1.0;
-        ib[P + t] = 1.0 / bet;
-        for (int j = 2; j <= n; ++j) {
-          const double cprev = (j == 2) ? 1.0 : c3;
-          const double aj = (j <= nz) ? c3 : -1.0;
-          const double bj = (j <= nz) ? bmid : 1.0;
-          const double g = cprev / bet;
-          bet = bj - aj * g;
-          if (bet == 0.0) throw Error(LESGO_ERR_NUMERIC, "tridag_array: zero pivot");
-          gm[(size_t)j * P + t] = g;
-          ib[(size_t)j * P + t] = 1.0 / bet;
+        // from the lower end to unknown m, from the upper end to m + 1 (rows
+        // 1 and n: b = -1, c = 1 and a = -1, b = 1), and the middle
+        const int m = n / 2;
+        double g[2];
+        for (int half = 0; half < 2; ++half) {
+          double h = -1.0;   // the end row's off-diagonal over its diagonal
+          gm[(size_t)(half ? n : 1) * P + t] = -1.0;
+          for (int q = 1; q <= (half ? n - 1 - m : m - 1); ++q) {
+            const double bet = bmid - c3 * h;
+            if (bet == 0.0) throw Error(LESGO_ERR_NUMERIC, "tridag_array: zero pivot");
+            h = c3 / bet;
+            gm[(size_t)(half ? n - q : 1 + q) * P + t] = h;
+          }
+          g[half] = h;
         }
+        if (g[0] * g[1] == 1.0) throw Error(LESGO_ERR_NUMERIC, "tridag_array: zero pivot");
+        gm[t] = 1.0 / (1.0 - g[0] * g[1]);
       }
     }
-    ibet_ = upload_vec(ib);
     tgam_ = upload_vec(gm);
   }
 
@@ -1792,7 +1794,10 @@ class Solver : public SolverBase {
     g.tw = rx_tw_; g.rtw = px_.rtw;
     return g;
   }
-  template <int NF> static void halve(SrcFields<R, NF>& s) { s.scale = s.isc ? (R)0.5 : (R)0.5 * s.scale; }
+  template <int NF> static void halve(SrcFields<R, NF>& s) {
+    s.scale = (R)0.5 * s.scale;
+    s.isc_mul = 0.5 * s.isc_mul;
+  }
   template <bool VO> static void halve(SrcVort<R, VO>& s) { s.c = (R)0.5 * s.c; }
 
   // The same transform as a tensor-core GEMM (k_xdft_tc): tiles of 128 rows,
@@ -2300,8 +2305,9 @@ class Solver : public SolverBase {
     const int nz = d_.nz, ny = d_.ny;
     const long long pl_s = (long long)ny * d_.K;
     const double c1 = 1.0 / ((double)d_.nx * d_.ny);
-    // scale 1/(nx ny tadv1 dt), the instance's step constant SC_PS
-    SrcFields<R, 3> su{{F_[LESGO_U], F_[LESGO_V], F_[LESGO_W]}, (R)0, 1, 1, d_.ld, kp_.plane, imf(nz), sc_d_, SC_PS};
+    // scale dz/(nx ny tadv1 dt): the instance's step constant SC_PS, and the
+    // dz that the solve's right-hand side takes (k_thomas)
+    SrcFields<R, 3> su{{F_[LESGO_U], F_[LESGO_V], F_[LESGO_W]}, (R)0, 1, 1, d_.ld, kp_.plane, imf(nz), sc_d_, SC_PS, d_.dz};
     xfwd<3>(su, d_.nx, ny, nz, specA_, px_, "press.xfwd");
     // the boundary planes (divtz at levels 1 and nz) on the second stream
     fork(3);
@@ -2314,33 +2320,16 @@ class Solver : public SolverBase {
     join(4);
     const long long vs = vol1_s_ * kp_.ninst;
     ThomasArgs ta;
-    ta.Hx = hspec_; ta.Hy = hspec_ + vs; ta.Hz = hspec_ + 2 * vs;
-    ta.Hb = hplane_; ta.Ht = hplane_ + pl_s;
-    ta.phat = phat_; ta.ibet = ibet_; ta.gam = tgam_;
+    const double* h = reinterpret_cast<const double*>(hspec_);
+    ta.Hx = h; ta.Hy = h + 2 * vs; ta.Hz = h + 4 * vs;
+    ta.Hb = reinterpret_cast<const double*>(hplane_);
+    ta.phat = reinterpret_cast<double*>(phat_); ta.g = tgam_;
     ta.kxw = kxw64_; ta.kyw = kyw64_;
-    ta.dz = d_.dz; ta.idz = 1.0 / d_.dz; ta.idz2 = 1.0 / (d_.dz * d_.dz);
+    ta.dz = d_.dz;
     ta.nz = nz; ta.ny = ny; ta.K = d_.K; ta.ninst = kp_.ninst;
+    const long long nblk = 2 * kp_.ninst + (pl_s * kp_.ninst + 7) / 8;   // mean modes, columns
     pre();
-    // The FP64 pipe bounds this solve on GB300.  With enough columns (a
-    // batch; measured: 17280 columns 20 % and 45056 columns 51 % faster
-    // than segmented) one thread sweeps each column in order, which does
-    // half the FP64 work of the segmented forms; with fewer columns (one
-    // 128^3 instance: 8320) the segmented forms keep the SMs busy: 16
-    // segments held in registers up to 192 unknowns, the looped form beyond.
-    // LESGO_THOMAS=seq|seg forces a form.
-    const long long ncol = pl_s * kp_.ninst;
-    const int nu = nz + 1;
-    const bool seq = thomas_mode_ == 1 || (thomas_mode_ == 0 && ncol >= 12288);
-    // four levels per register chunk: 96 registers a thread (164 with
-    // eight), so the sweep leaves room on the SMs for the other handles'
-    // kernels running beside it (the ensemble step measured 1 % shorter;
-    // the sweep alone takes the same time)
-    if (seq)
-      k_thomas_seq<4><<<(unsigned)((ncol + 127) / 128), 128, 0, st_>>>(ta);
-    else if (nu <= 192)
-      k_thomas_r<16, 8, 12><<<(unsigned)((ncol + 7) / 8), 128, 0, st_>>>(ta);
-    else
-      k_thomas<16, 16><<<(unsigned)((ncol + 15) / 16), 256, 0, st_>>>(ta);
+    k_thomas<4><<<(unsigned)nblk, 32, 0, st_>>>(ta);
     post("press.thomas", (double)pl_s * kp_.ninst * (4.0 * nz + 1.0) * sizeof(double2));
     // p, i kx p, i ky p at levels 1..nz-1; p at levels 0 and nz (phat holds nz+1 planes per instance)
     // p at levels 0 and nz on the second stream
@@ -2416,7 +2405,7 @@ class Solver : public SolverBase {
   R* fza_uv_ = nullptr;
   T2 *specA_ = nullptr, *specB_ = nullptr, *specC_ = nullptr;
   double2 *hspec_ = nullptr, *hplane_ = nullptr, *phat_ = nullptr;
-  double *ibet_ = nullptr, *tgam_ = nullptr;
+  double* tgam_ = nullptr;
   double *tacc_ = nullptr, *tw_d_ = nullptr, *prof_d_ = nullptr;
   double* sc_d_ = nullptr;                   // step constants [cap][SC_N]
   T2 *cvA_ = nullptr, *cvB_ = nullptr;       // convective-term spectra
@@ -2435,7 +2424,6 @@ class Solver : public SolverBase {
   size_t ybudget_ = sizeof(T2) == 16 ? 110 * 1024 : 48 * 1024;
   int ythreads_ = 256;   // y-pass block size (a multiple of the tile width)
   bool yshort_ = true;   // y-pass outputs without transforms where the operator allows (k_ypass)
-  int thomas_mode_ = 0;   // 0 by column count, 1 sequential, 2 segmented
   int dlog_cap_ = 0, dlog_every_ = 0;
   long long tacc_stride_ = 0;
   bool tavg_on_ = false;

@@ -62,7 +62,8 @@ struct InstMap {
 // Xf row loaders
 // ---------------------------------------------------------------------------
 // NF fields scaled by one constant, at levels lev0 + li*levstride.
-// With `isc` set, the scale is the instance's step constant isc[inst][isc_idx].
+// With `isc` set, the scale is isc_mul times the instance's step constant
+// isc[inst][isc_idx].
 template <typename R, int NF>
 struct SrcFields {
   using C = cplx<R>;   // the fields' complex pair type
@@ -73,10 +74,11 @@ struct SrcFields {
   InstMap im;
   const double* isc = nullptr;
   int isc_idx = 0;
+  double isc_mul = 1.0;
   __device__ __forceinline__ void load2(int n, int jy, int li, cplx<R>* v) const {
     const int inst = im.inst(li), lv = li - inst * im.nli;
     const long long off = inst * im.istr + (long long)(lev0 + lv * levstride) * plane + (long long)jy * ld + 2 * n;
-    const R scale = isc ? (R)isc[inst * SC_N + isc_idx] : this->scale;
+    const R scale = isc ? (R)(isc_mul * isc[inst * SC_N + isc_idx]) : this->scale;
 #pragma unroll
     for (int f = 0; f < NF; ++f) {
       cplx<R> a = *reinterpret_cast<const cplx<R>*>(p[f] + off);
