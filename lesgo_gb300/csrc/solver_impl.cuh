@@ -178,12 +178,19 @@ class SolverBase {
   virtual int diag_log_read(int id, double* out, int maxrows) = 0;
 };
 
-// Whether the convective term's 3/2-grid x-rows run as one pass
-// (k_convec_rows: c2r, products and r2c in shared memory) or as three
-// (xinv to six 3/2-grid fields in HBM, products, xfwd).  One pass for the
-// mixed and the double-word forms, three for the FP64 form, whose FP64
-// transforms leave the one-pass kernel slower (measured at 128^3: 8.06
-// against 7.87 ms per step); LESGO_CONVEC_ROWS=1 / 0 chooses for every form.
+// LESGO_RFFT=0: every pass on the run-time radix stages of fft_core.cuh.
+static bool rfft_enabled() {
+  const char* e = std::getenv("LESGO_RFFT");
+  return !e || std::strcmp(e, "0") != 0;
+}
+// Whether the convective term's 3/2-grid x-rows run as one pass (k_rx_rows
+// or k_convec_rows: c2r, products and r2c without 3/2-grid fields in memory)
+// or as three (xinv to six 3/2-grid fields in HBM, products, xfwd).  One
+// pass for the mixed and the double-word forms, three for the FP64 form,
+// which the FP64 pipe bounds either way: at 128^3 its three passes take 1.38
+// ms, k_convec_rows made the step 0.2 ms longer, and k_rx_rows in FP64, with
+// eight warps per SM to cover the FP64 latency, takes 1.84 ms.
+// LESGO_CONVEC_ROWS=1 / 0 chooses for every form.
 static bool convec_rows_enabled(int precision) {
   const char* e = std::getenv("LESGO_CONVEC_ROWS");
   if (e) return std::strcmp(e, "0") != 0;
@@ -220,7 +227,8 @@ template <> struct HostCvt<df64> {
 
 // Which arithmetic, row loaders and row epilogues have passes with the
 // transforms in registers (rfft_api.cuh).
-template <typename A> constexpr bool kRf = std::is_same<A, float>::value;
+template <typename A> constexpr bool kRf = std::is_same<A, float>::value || std::is_same<A, double>::value;
+template <typename A> constexpr bool kRfRows = std::is_same<A, float>::value;
 template <class S> constexpr bool kRxSrc = false;
 template <typename R> constexpr bool kRxSrc<SrcFields<R, 1>> = true;
 template <typename R> constexpr bool kRxSrc<SrcFields<R, 2>> = true;
@@ -312,8 +320,7 @@ class Solver : public SolverBase {
     if (const char* e = std::getenv("LESGO_YBUDGET")) ybudget_ = (size_t)std::max(8192, std::atoi(e));
     if (const char* e = std::getenv("LESGO_YTHREADS")) ythreads_ = std::atoi(e) == 128 ? 128 : 256;
     if (const char* e = std::getenv("LESGO_YSHORTCUT")) yshort_ = std::strcmp(e, "0") != 0;
-    // LESGO_RFFT=0: every pass on the run-time radix stages of fft_core.cuh
-    if (const char* e = std::getenv("LESGO_RFFT")) rf_ = std::strcmp(e, "0") != 0;
+    rf_ = rfft_enabled();
     use_graphs_ = graphs_allowed_;
     build_tables();
     // x-direction forward transforms as tensor-core GEMMs (FP32 transforms,
@@ -1680,7 +1687,7 @@ class Solver : public SolverBase {
         ry_twn_ = rf_table(r1, r2);
         ry_twm_ = rf_table(r1, 3 * r2 / 2);
       }
-      if (conv_rows_ && rxb_factors(d_.nx2 / 2, &r1, &r2)) rxb_tw_ = rf_table(r1, r2);
+      if (kRfRows<A> && conv_rows_ && rxb_factors(d_.nx2 / 2, &r1, &r2)) rxb_tw_ = rf_table(r1, r2);
     }
     // wavenumbers (fft.f90:130-160) for kx < nx/2 and every ky row
     const int ny = d_.ny, lh = d_.lh;
@@ -2191,7 +2198,7 @@ class Solver : public SolverBase {
   // The 3/2-grid x-rows of the convective term in one pass: the six padded
   // spectra of cvB_ in, the three products' x-spectra (nx/2 modes) into cvA_.
   void convec_rows(A cb) {
-    if constexpr (kRf<A>) {
+    if constexpr (kRfRows<A>) {
       if (rxb_tw_) {
         RxRowsGeom<A> rg;
         rg.ny2 = d_.ny2; rg.nz = d_.nz; rg.cz = 0; rg.err = err_ + 1;

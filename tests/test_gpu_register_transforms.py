@@ -65,3 +65,28 @@ def test_batch_of_uneven_rows_matches_alone(built_lib, grid):
             assert np.array_equal(s.get(f), b.get(iid, f)), (i, f)
         s.close()
     b.close()
+
+
+@pytest.mark.parametrize("grid", GRIDS, ids=IDS)
+def test_fp64_steps_match_oracle_and_radix(built_lib, monkeypatch, grid):
+    """The same passes in FP64: the form's 1e-10 against the oracle, and 1e-11
+    against the run-time radix passes (two FP64 transforms of at most 2^16
+    points differ by a few 1e-16, which four steps of dt = 1e-4 do not
+    amplify beyond the pressure's division by dt)."""
+    nx, ny, nz, kw = grid
+    kw = dict(nx=nx, ny=ny, Nz=nz, dt=1e-4, dyn_init=3, cs_count=3, **kw)
+    p, o, g = make_pair(**kw)
+    monkeypatch.setenv("LESGO_RFFT", "0")
+    _, _, r = make_pair(**kw)
+    for _ in range(4):
+        o.step()
+    for h in (g, r):
+        h.step(4)
+        h.sync()
+    for f in ("u", "v", "w", "p"):
+        e = rel_err(p, f, g.get(f), oracle_field(o, f))
+        assert e < 1e-10, (f, e)
+        e = rel_err(p, f, g.get(f), r.get(f))
+        assert e < 1e-11, (f, e)
+    g.close()
+    r.close()
