@@ -8,11 +8,25 @@ namespace lesgo {
 
 // ---------------------------------------------------------------------------
 // Wall models (wallstress.f90:107-255), evaluated in FP64 in every form.
-// Returns txz, tyz, dudz, dvdz at the wall level.
+// Returns txz, tyz, dudz, dvdz at the wall level.  wl holds the instance's
+// vonk / ln(dz/2 / z0) and 1 / (dz/2 ln(dz/2 / z0)) (made on the host): with
+// ustar = u_avg vonk / ln(..) the stress is -(vonk/ln)^2 u_avg u and the
+// gradient u / (dz/2 ln), without a logarithm or a division, whose FP64
+// instructions had taken most of a small grid's column sweep.
 // ---------------------------------------------------------------------------
 struct WallOut { double txz, tyz, dudz, dvdz; };
 
-__device__ __forceinline__ WallOut wall_bottom(const KP& kp, double zo, double u1f, double v1f, double u1, double v1) {
+__device__ __forceinline__ WallOut wall_equilibrium(const double* wl, double uf, double vf, double u, double v) {
+  const double u_avg = sqrt(uf * uf + vf * vf);
+  if (u_avg == 0.0) {   // the reference divides by u_avg
+    const double nan = __longlong_as_double(0x7ff8000000000000ll);
+    return WallOut{nan, nan, u == 0.0 ? 0.0 : nan, v == 0.0 ? 0.0 : nan};
+  }
+  const double c = wl[0] * wl[0] * u_avg;
+  return WallOut{c * uf, c * vf, u * wl[1], v * wl[1]};
+}
+
+__device__ __forceinline__ WallOut wall_bottom(const KP& kp, const double* wl, double u1f, double v1f, double u1, double v1) {
   WallOut o{0.0, 0.0, 0.0, 0.0};
   if (kp.lbc == 1) {                      // ws_dns_lbc (:131-148)
     o.dudz = (u1 - kp.ubot) / (0.5 * kp.dz);
@@ -20,19 +34,14 @@ __device__ __forceinline__ WallOut wall_bottom(const KP& kp, double zo, double u
     o.txz = -kp.nu_nd * o.dudz;
     o.tyz = -kp.nu_nd * o.dvdz;
   } else if (kp.lbc == 2) {               // ws_equilibrium_lbc (:171-219)
-    const double denom = log(0.5 * kp.dz / zo);
-    const double u_avg = sqrt(u1f * u1f + v1f * v1f);
-    const double ustar = u_avg * kp.vonk / denom;
-    const double c = -(ustar * ustar) / u_avg;
-    o.txz = c * u1f;
-    o.tyz = c * v1f;
-    o.dudz = (u1 == 0.0) ? 0.0 : ustar / (0.5 * kp.dz * kp.vonk) * u1 / u_avg;
-    o.dvdz = (v1 == 0.0) ? 0.0 : ustar / (0.5 * kp.dz * kp.vonk) * v1 / u_avg;
+    o = wall_equilibrium(wl, u1f, v1f, u1, v1);
+    o.txz = -o.txz;
+    o.tyz = -o.tyz;
   }
   return o;
 }
 
-__device__ __forceinline__ WallOut wall_top(const KP& kp, double zo, double utf, double vtf, double ut, double vt) {
+__device__ __forceinline__ WallOut wall_top(const KP& kp, const double* wl, double utf, double vtf, double ut, double vt) {
   WallOut o{0.0, 0.0, 0.0, 0.0};
   if (kp.ubc == 1) {                      // ws_dns_ubc (:151-168)
     o.dudz = (kp.utop - ut) / (0.5 * kp.dz);
@@ -40,14 +49,9 @@ __device__ __forceinline__ WallOut wall_top(const KP& kp, double zo, double utf,
     o.txz = -kp.nu_nd * o.dudz;
     o.tyz = -kp.nu_nd * o.dvdz;
   } else if (kp.ubc == 2) {               // ws_equilibrium_ubc (:222-255)
-    const double denom = log(0.5 * kp.dz / zo);
-    const double u_avg = sqrt(utf * utf + vtf * vtf);
-    const double ustar = u_avg * kp.vonk / denom;
-    const double c = (ustar * ustar) / u_avg;
-    o.txz = c * utf;
-    o.tyz = c * vtf;
-    o.dudz = (ut == 0.0) ? 0.0 : -ustar / (0.5 * kp.dz * kp.vonk) * ut / u_avg;
-    o.dvdz = (vt == 0.0) ? 0.0 : -ustar / (0.5 * kp.dz * kp.vonk) * vt / u_avg;
+    o = wall_equilibrium(wl, utf, vtf, ut, vt);
+    o.dudz = -o.dudz;
+    o.dvdz = -o.dvdz;
   }
   return o;
 }
@@ -55,8 +59,17 @@ __device__ __forceinline__ WallOut wall_top(const KP& kp, double zo, double utf,
 // ---------------------------------------------------------------------------
 // Fused z-column sweep: ddz_uv/ddz_w (derivatives.f90:214-311), the wall
 // values, calc_Sij (sgs_stag_util.f90:467-634), |S|, Nu_t and the stresses
-// (sgs_stag_util.f90:223-428).  One thread owns an (i,j) column over a
-// chunk of levels [k0, k1) and recomputes the level above the chunk.
+// (sgs_stag_util.f90:223-428).  One thread owns two neighbouring columns over
+// a chunk of levels [k0, k1) and recomputes the level above the chunk; a
+// level's loads are issued under the arithmetic of the level below.  The host
+// picks the chunk so that small grids too give every SM several warps.
+// Measured, us per launch against one column per thread, 16 levels and the
+// wall law with its logarithm and divisions in the sweep: 32^3 FP64 25 (80),
+// 48^3 mixed 12 (31), 128^3 mixed 42 (55; unique bytes 24), 256x256x192 mixed
+// 178 (244; 142), 128^3 FP64 242 (273).
+//
+// Bound by HBM in FP32 at large grids, by the FP64 pipe in FP64 (S is carried
+// doubled, T = 2 S, which saves the halvings).
 // FLAGS: COL_DDZ compute+store dudz/dvdz/dwdz and the wall values (else
 //        they are read from their fields); COL_STORE_S store S_ij;
 //        COL_TAU emit the stresses; COL_READ_S read S_ij instead of
@@ -72,19 +85,19 @@ struct ColArgs {
   R *Cs, *txx, *txy, *txz, *tyy, *tyz, *tzz;
   const R *wb_u, *wb_v, *wt_u, *wt_v;   // test-filtered wall planes
   KP kp;
-  double delta2;
+  FastDiv fnx2;                         // by nx / 2
+  double nu_scale;                      // delta^2 / sqrt(2): Nu_t = nu_scale Cs^2 |T|
   int chunk;
 };
 
-template <typename R>
-struct Sij { R s11, s12, s13, s22, s23, s33; };
-
 template <typename R, int FLAGS>
-__global__ void __launch_bounds__(256) k_column(ColArgs<R> a) {
+__global__ void __launch_bounds__(128) k_column(ColArgs<R> a) {
+  using C = cplx<R>;
   const KP& kp = a.kp;
   const int col = blockIdx.x * blockDim.x + threadIdx.x;
-  if (col >= kp.nx * kp.ny) return;
-  const int j = col / kp.nx, i = col - j * kp.nx;
+  const int nx2 = kp.nx / 2;
+  if (col >= nx2 * kp.ny) return;
+  const int j = a.fnx2.div(col), i = 2 * (col - j * nx2);
   const int nz = kp.nz;
   const int k0 = 1 + blockIdx.y * a.chunk;
   if (k0 > nz) return;
@@ -93,144 +106,181 @@ __global__ void __launch_bounds__(256) k_column(ColArgs<R> a) {
   const long long P = kp.plane;
   const long long cw = inst * P + (long long)j * kp.ld + i;          // wall planes (ld, ny) per instance
   const long long c0 = inst * kp.istride + (long long)j * kp.ld + i;  // 3-D fields
-  const double zo = kp.zo_i[inst];
   const bool cs_fill = (kp.iflags[inst] & IF_CSFILL) != 0;
   const R inv_dz = (R)kp.idz;
   const R h = (R)0.5;
+  auto ld = [](const R* p) { return *reinterpret_cast<const C*>(p); };
+  auto st = [](R* p, C v) { *reinterpret_cast<C*>(p) = v; };
+  const C z2 = mkc((R)0, (R)0);
 
   // wall values (needed at k = 1 and k = nz)
-  WallOut wb{0, 0, 0, 0}, wt{0, 0, 0, 0};
+  C wbz[4] = {z2, z2, z2, z2}, wtz[4] = {z2, z2, z2, z2};   // txz, tyz, dudz, dvdz
   if (FLAGS & COL_DDZ) {
+    const double* wl = kp.wall_i + 2 * inst;
+    auto pack = [&](const WallOut& x, const WallOut& y, C* o) {
+      o[0] = mkc((R)x.txz, (R)y.txz); o[1] = mkc((R)x.tyz, (R)y.tyz);
+      o[2] = mkc((R)x.dudz, (R)y.dudz); o[3] = mkc((R)x.dvdz, (R)y.dvdz);
+    };
     if (k0 == 1) {
-      double uf = 0, vf = 0;
-      if (kp.lbc == 2) { uf = a.wb_u[cw]; vf = a.wb_v[cw]; }
-      wb = wall_bottom(kp, zo, uf, vf, (double)a.u[P + c0], (double)a.v[P + c0]);
+      C uf = z2, vf = z2;
+      if (kp.lbc == 2) { uf = ld(a.wb_u + cw); vf = ld(a.wb_v + cw); }
+      const C u = ld(a.u + P + c0), v = ld(a.v + P + c0);
+      pack(wall_bottom(kp, wl, (double)uf.x, (double)vf.x, (double)u.x, (double)v.x),
+           wall_bottom(kp, wl, (double)uf.y, (double)vf.y, (double)u.y, (double)v.y), wbz);
     }
     if (k1 >= nz) {
-      double uf = 0, vf = 0;
-      if (kp.ubc == 2) { uf = a.wt_u[cw]; vf = a.wt_v[cw]; }
-      wt = wall_top(kp, zo, uf, vf, (double)a.u[(nz - 1) * P + c0], (double)a.v[(nz - 1) * P + c0]);
+      C uf = z2, vf = z2;
+      if (kp.ubc == 2) { uf = ld(a.wt_u + cw); vf = ld(a.wt_v + cw); }
+      const C u = ld(a.u + (nz - 1) * P + c0), v = ld(a.v + (nz - 1) * P + c0);
+      pack(wall_top(kp, wl, (double)uf.x, (double)vf.x, (double)u.x, (double)v.x),
+           wall_top(kp, wl, (double)uf.y, (double)vf.y, (double)u.y, (double)v.y), wtz);
     }
   }
-  auto uz_at = [&](int k) -> R {
+
+  // what a level reads: the six gradients (or S), with COL_DDZ u, v and the w
+  // above, else the z gradients; Cs
+  struct Level { C g[6], z[3], cs; };
+  auto load = [&](int k, Level& l) {
     const long long q = k * P + c0;
-    if (!(FLAGS & COL_DDZ)) return a.dudz[q];
-    if (k == 1) return (R)wb.dudz;
-    if (k == nz) return (R)wt.dudz;
-    return inv_dz * (a.u[q] - a.u[q - P]);
-  };
-  auto vz_at = [&](int k) -> R {
-    const long long q = k * P + c0;
-    if (!(FLAGS & COL_DDZ)) return a.dvdz[q];
-    if (k == 1) return (R)wb.dvdz;
-    if (k == nz) return (R)wt.dvdz;
-    return inv_dz * (a.v[q] - a.v[q - P]);
-  };
-  auto wz_at = [&](int k) -> R {
-    const long long q = k * P + c0;
-    if (k >= nz) return (R)0;
-    if (!(FLAGS & COL_DDZ)) return a.dwdz[q];
-    return inv_dz * (a.w[q + P] - a.w[q]);
+    if (FLAGS & COL_READ_S) {
+      l.g[0] = ld(a.S11 + q); l.g[1] = ld(a.S12 + q); l.g[2] = ld(a.S13 + q);
+      l.g[3] = ld(a.S22 + q); l.g[4] = ld(a.S23 + q); l.g[5] = ld(a.S33 + q);
+    } else {
+      l.g[0] = ld(a.dudx + q); l.g[1] = ld(a.dudy + q); l.g[2] = ld(a.dvdx + q);
+      l.g[3] = ld(a.dvdy + q); l.g[4] = ld(a.dwdx + q); l.g[5] = ld(a.dwdy + q);
+      if (FLAGS & COL_DDZ) {
+        l.z[0] = ld(a.u + q); l.z[1] = ld(a.v + q);
+        l.z[2] = k < nz ? ld(a.w + q + P) : z2;
+      } else {
+        l.z[0] = ld(a.dudz + q); l.z[1] = ld(a.dvdz + q);
+        l.z[2] = k < nz ? ld(a.dwdz + q) : z2;
+      }
+    }
+    if ((FLAGS & COL_TAU) && !cs_fill) l.cs = ld(a.Cs + q);
   };
 
-  // derivative window: values at level k-1 (p*) and k (c*)
-  R pux = 0, puy = 0, pvx = 0, pvy = 0, pwx = 0, pwy = 0, pwz = 0;
-  if (!(FLAGS & COL_READ_S) && k0 > 1) {
-    const long long q = (k0 - 1) * P + c0;
-    pux = a.dudx[q]; puy = a.dudy[q]; pvx = a.dvdx[q]; pvy = a.dvdy[q];
-    pwx = a.dwdx[q]; pwy = a.dwdy[q]; pwz = wz_at(k0 - 1);
+  // the level below: gradients, and u, v; w of this level
+  C pg[4] = {z2, z2, z2, z2}, pwx = z2, pwy = z2, pwz = z2, pu = z2, pv = z2, pw = z2;
+  if (!(FLAGS & COL_READ_S)) {
+    if (k0 > 1) {
+      const long long q = (k0 - 1) * P + c0;
+      pg[0] = ld(a.dudx + q); pg[1] = ld(a.dudy + q); pg[2] = ld(a.dvdx + q); pg[3] = ld(a.dvdy + q);
+      pwx = ld(a.dwdx + q); pwy = ld(a.dwdy + q);
+      if (FLAGS & COL_DDZ) {
+        pu = ld(a.u + q); pv = ld(a.v + q);
+        pw = ld(a.w + q + P);
+        pwz = cscale(csub(pw, ld(a.w + q)), inv_dz);
+      } else {
+        pwz = ld(a.dwdz + q);
+      }
+    } else if (FLAGS & COL_DDZ) {
+      pw = ld(a.w + P + c0);
+    }
   }
-  Sij<R> Sp{0, 0, 0, 0, 0, 0};
-  R Np = 0;
+  C Tp[6] = {z2, z2, z2, z2, z2, z2}, Np = z2;   // T and Nu_t of the level below
   const int kend = min(k1, nz);
+  Level next;
+  load(k0, next);
+#pragma unroll 1
   for (int k = k0; k <= kend; ++k) {
+    const Level l = next;
+    if (k < kend) load(k + 1, next);
     const long long q = k * P + c0;
-    Sij<R> S;
+    C T[6];   // 11 12 13 22 23 33 of 2 S, with COL_READ_S of S
+    constexpr R kF = (FLAGS & COL_READ_S) ? (R)2 : (R)1;   // 2 S = kF T
     if (FLAGS & COL_READ_S) {
-      S = Sij<R>{a.S11[q], a.S12[q], a.S13[q], a.S22[q], a.S23[q], a.S33[q]};
+#pragma unroll
+      for (int s = 0; s < 6; ++s) T[s] = l.g[s];
     } else {
-      const R ux = a.dudx[q], uy = a.dudy[q], vx = a.dvdx[q], vy = a.dvdy[q];
-      const R wx = a.dwdx[q], wy = a.dwdy[q];
-      const R uz = uz_at(k), vz = vz_at(k), wz = wz_at(k);
+      const C ux = l.g[0], uy = l.g[1], vx = l.g[2], vy = l.g[3], wx = l.g[4], wy = l.g[5];
+      C uz = l.z[0], vz = l.z[1], wz = l.z[2];
+      if (FLAGS & COL_DDZ) {
+        uz = k == 1 ? wbz[2] : k == nz ? wtz[2] : cscale(csub(l.z[0], pu), inv_dz);
+        vz = k == 1 ? wbz[3] : k == nz ? wtz[3] : cscale(csub(l.z[1], pv), inv_dz);
+        wz = k < nz ? cscale(csub(l.z[2], pw), inv_dz) : z2;
+      }
       if (k == 1) {
+        T[0] = cadd(ux, ux); T[1] = cadd(uy, vx); T[3] = cadd(vy, vy);
         if (kp.lbc == 0) {
-          S = Sij<R>{ux, h * (uy + vx), h * (uz + wx), vy, h * (vz + wy), h * (wz + (R)0)};
+          T[2] = cadd(uz, wx); T[4] = cadd(vz, wy); T[5] = wz;
         } else {
-          const R wx2 = h * (wx + a.dwdx[q + P]);
-          const R wy2 = h * (wy + a.dwdy[q + P]);
-          S = Sij<R>{ux, h * (uy + vx), h * (uz + wx2), vy, h * (vz + wy2), wz};
+          T[2] = cadd(uz, cscale(cadd(wx, ld(a.dwdx + q + P)), h));
+          T[4] = cadd(vz, cscale(cadd(wy, ld(a.dwdy + q + P)), h));
+          T[5] = cadd(wz, wz);
         }
       } else if (k == nz) {
+        T[0] = cadd(pg[0], pg[0]); T[1] = cadd(pg[1], pg[2]); T[3] = cadd(pg[3], pg[3]);
         if (kp.ubc == 0) {
-          S = Sij<R>{pux, h * (puy + pvx), h * (uz + wx), pvy, h * (vz + wy), h * (pwz + (R)0)};
+          T[2] = cadd(uz, wx); T[4] = cadd(vz, wy); T[5] = pwz;
         } else {
-          const R wx2 = h * (pwx + wx), wy2 = h * (pwy + wy);
-          S = Sij<R>{pux, h * (puy + pvx), h * (uz + wx2), pvy, h * (vz + wy2), pwz};
+          T[2] = cadd(uz, cscale(cadd(pwx, wx), h));
+          T[4] = cadd(vz, cscale(cadd(pwy, wy), h));
+          T[5] = cadd(pwz, pwz);
         }
       } else {
-        const R uyy = uy + puy, vxx = vx + pvx;
-        S = Sij<R>{h * (ux + pux), (R)0.25 * (uyy + vxx), h * (uz + wx), h * (vy + pvy), h * (vz + wy), h * (wz + pwz)};
+        T[0] = cadd(ux, pg[0]);
+        T[1] = cscale(cadd(cadd(uy, pg[1]), cadd(vx, pg[2])), h);
+        T[2] = cadd(uz, wx);
+        T[3] = cadd(vy, pg[3]);
+        T[4] = cadd(vz, wy);
+        T[5] = cadd(wz, pwz);
       }
       if (k < k1) {
         if (FLAGS & COL_STORE_S) {
-          a.S11[q] = S.s11; a.S12[q] = S.s12; a.S13[q] = S.s13;
-          a.S22[q] = S.s22; a.S23[q] = S.s23; a.S33[q] = S.s33;
+          st(a.S11 + q, cscale(T[0], h)); st(a.S12 + q, cscale(T[1], h)); st(a.S13 + q, cscale(T[2], h));
+          st(a.S22 + q, cscale(T[3], h)); st(a.S23 + q, cscale(T[4], h)); st(a.S33 + q, cscale(T[5], h));
         }
         if (FLAGS & COL_DDZ) {
-          a.dudz[q] = uz;
-          a.dvdz[q] = vz;
-          if (k <= nz - 1) a.dwdz[q] = wz;
-          if (k == 1) { a.txz[q] = (R)wb.txz; a.tyz[q] = (R)wb.tyz; }
-          if (k == nz) { a.txz[q] = (R)wt.txz; a.tyz[q] = (R)wt.tyz; }
+          st(a.dudz + q, uz);
+          st(a.dvdz + q, vz);
+          if (k <= nz - 1) st(a.dwdz + q, wz);
+          if (k == 1) { st(a.txz + q, wbz[0]); st(a.tyz + q, wbz[1]); }
+          if (k == nz) { st(a.txz + q, wtz[0]); st(a.tyz + q, wtz[1]); }
         }
       }
-      pux = ux; puy = uy; pvx = vx; pvy = vy; pwx = wx; pwy = wy; pwz = wz;
+      pg[0] = ux; pg[1] = uy; pg[2] = vx; pg[3] = vy; pwx = wx; pwy = wy; pwz = wz;
+      if (FLAGS & COL_DDZ) { pu = l.z[0]; pv = l.z[1]; pw = l.z[2]; }
     }
     if (FLAGS & COL_TAU) {
-      R cs;
+      C cs = l.cs;
       if (cs_fill) {
-        cs = (R)0.03;
-        if (k < k1) a.Cs[q] = cs;
-      } else {
-        cs = a.Cs[q];
+        cs = mkc((R)0.03, (R)0.03);
+        if (k < k1) st(a.Cs + q, cs);
       }
-      const R Sm = sqrt((R)2 * (S.s11 * S.s11 + S.s22 * S.s22 + S.s33 * S.s33 +
-                                (R)2 * (S.s12 * S.s12 + S.s13 * S.s13 + S.s23 * S.s23)));
-      const R Nu = Sm * cs * (R)a.delta2;
+      auto nu_t = [&](R t0, R t1, R t2, R t3, R t4, R t5, R c) {
+        const R d = t0 * t0 + t3 * t3 + t5 * t5, o = t1 * t1 + t2 * t2 + t4 * t4;
+        return sqrt(d + (R)2 * o) * (c * (kF * (R)a.nu_scale));
+      };
+      const C Nu = mkc(nu_t(T[0].x, T[1].x, T[2].x, T[3].x, T[4].x, T[5].x, cs.x),
+                       nu_t(T[0].y, T[1].y, T[2].y, T[3].y, T[4].y, T[5].y, cs.y));
       const int m = k - 1;   // emit the stresses of level m = k-1
       if (m >= k0 && m <= nz - 1) {
         const long long qm = q - P;
         const R nu = (R)kp.nu;
-        if (m == nz - 1) {
-          if (kp.ubc == 0) {
-            const R c = h * (Np + Nu) + nu, c2 = (R)2 * (Np + nu);
-            a.txx[qm] = -c * (Sp.s11 + S.s11); a.txy[qm] = -c * (Sp.s12 + S.s12);
-            a.tyy[qm] = -c * (Sp.s22 + S.s22); a.tzz[qm] = -c * (Sp.s33 + S.s33);
-            a.txz[qm] = -c2 * Sp.s13; a.tyz[qm] = -c2 * Sp.s23;
-          } else {
-            const R c = (R)-2 * (Nu + nu), c2 = (R)-2 * (Np + nu);
-            a.txx[qm] = c * S.s11; a.txy[qm] = c * S.s12; a.tyy[qm] = c * S.s22; a.tzz[qm] = c * S.s33;
-            a.txz[qm] = c2 * Sp.s13; a.tyz[qm] = c2 * Sp.s23;
-          }
-        } else if (m == 1) {
-          if (kp.lbc == 0) {
-            const R c = h * (Np + Nu) + nu;
-            a.txx[qm] = -c * (Sp.s11 + S.s11); a.txy[qm] = -c * (Sp.s12 + S.s12);
-            a.tyy[qm] = -c * (Sp.s22 + S.s22); a.tzz[qm] = -c * (Sp.s33 + S.s33);
-          } else {
-            const R c = (R)-2 * (Np + nu);
-            a.txx[qm] = c * Sp.s11; a.txy[qm] = c * Sp.s12; a.tyy[qm] = c * Sp.s22; a.tzz[qm] = c * Sp.s33;
-          }
+        auto mul = [](C x, C y) { return mkc(x.x * y.x, x.y * y.y); };
+        // -2 (Nu + nu) S = -(Nu + nu) T; across a cell -(Nu_a + Nu_b)/2 - nu
+        // times the sum of the S, half of it times the sum of the T
+        const C own = mkc(-kF * Np.x - kF * nu, -kF * Np.y - kF * nu);
+        C c, s[4];
+        if (m == nz - 1 && kp.ubc != 0) {
+          c = mkc(-kF * Nu.x - kF * nu, -kF * Nu.y - kF * nu);
+          s[0] = T[0]; s[1] = T[1]; s[2] = T[3]; s[3] = T[5];
+        } else if (m == 1 && m != nz - 1 && kp.lbc != 0) {
+          c = own;
+          s[0] = Tp[0]; s[1] = Tp[1]; s[2] = Tp[3]; s[3] = Tp[5];
         } else {
-          const R c = -h * (Np + Nu), c2 = (R)-2 * Np, c3 = (R)-2 * nu * h, c4 = (R)-2 * nu;
-          a.txx[qm] = (c + c3) * (Sp.s11 + S.s11); a.txy[qm] = (c + c3) * (Sp.s12 + S.s12);
-          a.tyy[qm] = (c + c3) * (Sp.s22 + S.s22); a.tzz[qm] = (c + c3) * (Sp.s33 + S.s33);
-          a.txz[qm] = (c2 + c4) * Sp.s13; a.tyz[qm] = (c2 + c4) * Sp.s23;
+          const R hn = h * kF * nu, qf = (R)-0.25 * kF;
+          c = mkc(qf * (Np.x + Nu.x) - hn, qf * (Np.y + Nu.y) - hn);
+          s[0] = cadd(Tp[0], T[0]); s[1] = cadd(Tp[1], T[1]); s[2] = cadd(Tp[3], T[3]); s[3] = cadd(Tp[5], T[5]);
         }
+        st(a.txx + qm, mul(c, s[0])); st(a.txy + qm, mul(c, s[1]));
+        st(a.tyy + qm, mul(c, s[2])); st(a.tzz + qm, mul(c, s[3]));
+        if (m > 1) { st(a.txz + qm, mul(own, Tp[2])); st(a.tyz + qm, mul(own, Tp[4])); }
       }
       Np = Nu;
     }
-    Sp = S;
+#pragma unroll
+    for (int s = 0; s < 6; ++s) Tp[s] = T[s];
   }
 }
 
@@ -279,10 +329,10 @@ __global__ void k_wall(const R* u, const R* v, const R* wb_u, const R* wb_v, con
   const long long cw = inst * P + (long long)j * kp.ld + i;
   const long long c0 = inst * kp.istride + (long long)j * kp.ld + i;
   const int nz = kp.nz;
-  const double zo = kp.zo_i[inst];
-  WallOut b = wall_bottom(kp, zo, kp.lbc == 2 ? (double)wb_u[cw] : 0.0, kp.lbc == 2 ? (double)wb_v[cw] : 0.0,
+  const double* wl = kp.wall_i + 2 * inst;
+  WallOut b = wall_bottom(kp, wl, kp.lbc == 2 ? (double)wb_u[cw] : 0.0, kp.lbc == 2 ? (double)wb_v[cw] : 0.0,
                           (double)u[P + c0], (double)v[P + c0]);
-  WallOut t = wall_top(kp, zo, kp.ubc == 2 ? (double)wt_u[cw] : 0.0, kp.ubc == 2 ? (double)wt_v[cw] : 0.0,
+  WallOut t = wall_top(kp, wl, kp.ubc == 2 ? (double)wt_u[cw] : 0.0, kp.ubc == 2 ? (double)wt_v[cw] : 0.0,
                        (double)u[(nz - 1) * P + c0], (double)v[(nz - 1) * P + c0]);
   txz[P + c0] = (R)b.txz; tyz[P + c0] = (R)b.tyz; dudz[P + c0] = (R)b.dudz; dvdz[P + c0] = (R)b.dvdz;
   const long long qt = nz * P + c0;

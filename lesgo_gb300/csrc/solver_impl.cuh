@@ -302,12 +302,14 @@ class Solver : public SolverBase {
     build_thomas_pivots();
     err_ = alloc<int>(2);   // [0] zero pivot, [1] a bulk-copy wait that gave up
     zo_d_ = alloc<double>(cap_);
+    wall_d_ = alloc<double>(2 * cap_);
     flags_d_ = alloc<int>(cap_);
     // pinned staging ring for the per-step uploads (flags, averaging actions):
     // copies from pageable memory would wait for the stream every step
     CK(cudaMallocHost(&ring_h_, (size_t)kRing * cap_ * sizeof(int)));
     for (auto& e : ring_ev_) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     kp_.zo_i = zo_d_;
+    kp_.wall_i = wall_d_;
     kp_.iflags = flags_d_;
     sc_d_ = alloc<double>((long long)SC_N * cap_);
     cflmax_d_ = alloc<unsigned long long>(3LL * cap_);
@@ -1264,6 +1266,13 @@ class Solver : public SolverBase {
     std::vector<double> zo(cap_, d_.p.zo);
     for (size_t s = 0; s < slots_.size(); ++s) zo[s] = slots_[s].spec.zo;
     CK(cudaMemcpyAsync(zo_d_, zo.data(), cap_ * sizeof(double), cudaMemcpyHostToDevice, st_));
+    std::vector<double> wall(2 * cap_);
+    for (int s = 0; s < cap_; ++s) {
+      const double denom = std::log(0.5 * d_.dz / zo[s]);
+      wall[2 * s] = d_.p.vonk / denom;
+      wall[2 * s + 1] = 1.0 / (0.5 * d_.dz * denom);
+    }
+    CK(cudaMemcpyAsync(wall_d_, wall.data(), wall.size() * sizeof(double), cudaMemcpyHostToDevice, st_));
     CK(cudaStreamSynchronize(st_));
   }
 
@@ -2112,13 +2121,16 @@ class Solver : public SolverBase {
     a.tyy = F_[LESGO_TYY]; a.tyz = F_[LESGO_TYZ]; a.tzz = F_[LESGO_TZZ];
     a.wb_u = wall_[0]; a.wb_v = wall_[1]; a.wt_u = wall_[2]; a.wt_v = wall_[3];
     a.kp = kp_;
-    a.delta2 = d_.delta * d_.delta;
-    a.chunk = 16;
-    const int ncol = d_.nx * d_.ny;
-    dim3 grid((ncol + 255) / 256, (d_.nz + a.chunk - 1) / a.chunk, kp_.ninst);
+    a.nu_scale = d_.delta * d_.delta * std::sqrt(0.5);
+    a.fnx2 = FastDiv((unsigned)(d_.nx / 2));
+    const int ncol = d_.nx * d_.ny, npair = ncol / 2;
+    // levels per thread: about sixteen warps per SM, 4 to 16 levels (each
+    // chunk reads one level more)
+    a.chunk = (int)std::min(16LL, std::max(4LL, (long long)npair * d_.nz * kp_.ninst / (32 * 16 * 152)));
+    dim3 grid((npair + 127) / 128, (d_.nz + a.chunk - 1) / a.chunk, kp_.ninst);
     const int nrw = (FLAGS & COL_READ_S) ? 13 : (FLAGS & COL_TAU) ? 19 : 18;
     pre();
-    k_column<R, FLAGS><<<grid, 256, 0, st_>>>(a);
+    k_column<R, FLAGS><<<grid, 128, 0, st_>>>(a);
     post((FLAGS & COL_READ_S) ? "sgs_column.tau" : (FLAGS & COL_TAU) ? "sgs_column" : "sgs_column.sij",
          (double)nrw * ncol * d_.nz * kp_.ninst * sizeof(R));
   }
@@ -2436,7 +2448,7 @@ class Solver : public SolverBase {
   bool tavg_on_ = false;
   int ta_nstart_ = 1, ta_nend_ = 50000, ta_nskip_ = 100;
   int* err_ = nullptr;
-  double* zo_d_ = nullptr;
+  double *zo_d_ = nullptr, *wall_d_ = nullptr;
   int* flags_d_ = nullptr;
   double *diag_part_ = nullptr, *diag_out_ = nullptr;
   double* staging_ = nullptr;

@@ -18,6 +18,7 @@ struct KP {
   long long istride;         // elements between instances of a field: (nz+1)*plane
   long long istride_big;     // same on the 3/2 grid
   const double* zo_i;        // per-instance roughness length
+  const double* wall_i;      // per-instance constants of the wall law, [inst][2] (wall_equilibrium)
   const int* iflags;         // per-instance step flags (IF_*)
   const double* sc;          // per-instance step constants [inst][SC_N] (SC_*)
   FastDiv fnx, fny, fnz;     // by nx, ny, nz (point-index decomposition)
