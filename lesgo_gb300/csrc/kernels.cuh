@@ -702,28 +702,35 @@ __global__ void __launch_bounds__(32) k_thomas(ThomasArgs a) {
 }
 
 // press_stag_array.f90:284-288 dpdz + main.f90:321-326 + forcing.f90:184-243
-// (FUSED: RHSz -= dpdz, project w, boundary conditions) or just dpdz.
+// (FUSED: RHSz -= dpdz, project w, boundary conditions) or just dpdz.  Bound
+// by HBM: a thread has two neighbouring points (8 or 16 bytes per access;
+// 256x256x192 mixed 58 us against 76 with one point, unique bytes 37).
 template <typename R, bool FUSED>
-__global__ void k_wproj(const R* __restrict__ p, R* dpdz, R* RHSz, R* u, R* v, R* w, KP kp) {
+__global__ void __launch_bounds__(256) k_wproj(const R* __restrict__ p, R* dpdz, R* RHSz, R* u, R* v, R* w, KP kp) {
+  using C = cplx<R>;
   const long long n = (long long)kp.nx * kp.ny * kp.nz * kp.ninst;
-  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  const long long t = 2 * (blockIdx.x * (long long)blockDim.x + threadIdx.x);   // nx is even: a pair is in one row
   if (t >= n) return;
   const PtIdx x = pt_index(t, kp);
   const int k = x.k;
   const long long P = kp.plane;
   const long long q = x.q;
+  auto ld = [](const R* a) { return *reinterpret_cast<const C*>(a); };
+  auto st = [](R* a, C b) { *reinterpret_cast<C*>(a) = b; };
   // (p(k) - p(k-1)) / dz as a multiply by 1/dz: within an ulp of the
   // division, which is a long instruction sequence in FP64 on this part
-  const R d = (p[q] - p[q - P]) * (R)kp.idz;
-  if (!FUSED) { dpdz[q] = d; return; }
-  RHSz[q] = RHSz[q] - d;
+  const C d = cscale(csub(ld(p + q), ld(p + q - P)), (R)kp.idz);
+  if (!FUSED) { st(dpdz + q, d); return; }
   const int nz = kp.nz;
-  const double* c = kp.sc + x.inst * SC_N;
-  if (k >= 2 && k <= nz - 1) w[q] = w[q] + (R)c[SC_DT] * (-(R)c[SC_T1] * d);
-  if (k == 1) w[q] = (R)0;
-  if (k == nz) {
-    w[q] = (R)0;
-    if (kp.ubc == 0) { u[q] = u[q - P]; v[q] = v[q - P]; }
+  const C r = ld(RHSz + q), w0 = ld(w + q);
+  st(RHSz + q, csub(r, d));
+  if (k >= 2 && k <= nz - 1) {
+    const double* c = kp.sc + x.inst * SC_N;
+    const R dt = (R)c[SC_DT], t1 = (R)c[SC_T1];
+    st(w + q, mkc(w0.x + dt * (-t1 * d.x), w0.y + dt * (-t1 * d.y)));
+  } else {
+    st(w + q, mkc((R)0, (R)0));
+    if (k == nz && kp.ubc == 0) { st(u + q, ld(u + q - P)); st(v + q, ld(v + q - P)); }
   }
 }
 
@@ -1343,36 +1350,48 @@ namespace lesgo {
 // Time step on the device.  k_cfl_max: per instance the maxima of |u|, |v|,
 // |w| over x < nx and levels 1..nz-1 (cfl_util.f90:70-111), folded into
 // mx[inst][3] as the bit patterns of non-negative doubles (ordered like the
-// values).  Grid (blocks, instances).
+// values).  Grid (blocks, instances).  The maxima are kept in the fields'
+// own type, two points a step (in FP64, their conversions and comparisons
+// had made this pass of three fields FP64-bound: 45 us against 166 at
+// 256x256x192).
 // ---------------------------------------------------------------------------
 template <typename R>
 __global__ void __launch_bounds__(256) k_cfl_max(const R* u, const R* v, const R* w, KP kp,
                                                  unsigned long long* mx) {
-  __shared__ double sh[3][256];
+  using C = cplx<R>;
+  __shared__ R sh[3][8];
   const int inst = blockIdx.y;
-  const long long m = (long long)kp.nx * kp.ny * (kp.nz - 1);
+  const long long m = (long long)kp.nx * kp.ny * (kp.nz - 1) / 2;   // pairs
   const long long base = inst * kp.istride + kp.plane;
-  double au = 0.0, av = 0.0, aw = 0.0;
+  R mxv[3] = {(R)0, (R)0, (R)0};
+#pragma unroll 4
   for (long long t = blockIdx.x * 256LL + threadIdx.x; t < m; t += (long long)gridDim.x * 256) {
-    const int ti = (int)t;
+    const int ti = 2 * (int)t;
     const int r = kp.fnx.div(ti);
     const int i = ti - r * kp.nx;
     const int k = kp.fny.div(r);     // 0 .. nz-2 (level k + 1)
     const int j = r - k * kp.ny;
     const long long q = base + k * kp.plane + (long long)j * kp.ld + i;
-    au = fmax(au, fabs((double)u[q]));
-    av = fmax(av, fabs((double)v[q]));
-    aw = fmax(aw, fabs((double)w[q]));
+    const R* f[3] = {u, v, w};
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const C a = *reinterpret_cast<const C*>(f[c] + q);
+      mxv[c] = fmax(mxv[c], fmax(fabs(a.x), fabs(a.y)));
+    }
   }
-  sh[0][threadIdx.x] = au; sh[1][threadIdx.x] = av; sh[2][threadIdx.x] = aw;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) mxv[c] = fmax(mxv[c], __shfl_xor_sync(0xffffffffu, mxv[c], d));
+    if ((threadIdx.x & 31) == 0) sh[c][threadIdx.x >> 5] = mxv[c];
+  }
   __syncthreads();
-  for (int st = 128; st > 0; st >>= 1) {
-    if (threadIdx.x < st)
-      for (int c = 0; c < 3; ++c) sh[c][threadIdx.x] = fmax(sh[c][threadIdx.x], sh[c][threadIdx.x + st]);
-    __syncthreads();
+  if (threadIdx.x < 3) {
+    R r = sh[threadIdx.x][0];
+#pragma unroll
+    for (int d = 1; d < 8; ++d) r = fmax(r, sh[threadIdx.x][d]);
+    atomicMax(&mx[inst * 3 + threadIdx.x], (unsigned long long)__double_as_longlong((double)r));
   }
-  if (threadIdx.x < 3)
-    atomicMax(&mx[inst * 3 + threadIdx.x], (unsigned long long)__double_as_longlong(sh[threadIdx.x][0]));
 }
 
 // Start of a step, one thread per instance: with cfl_mode, dt from the maxima

@@ -2371,12 +2371,9 @@ class Solver : public SolverBase {
     join(6);
     const long long n = (long long)d_.nx * ny * nz * kp_.ninst;
     pre();
-    if (fused)
-      k_wproj<R, true><<<grid1(n), 256, 0, st_>>>(F_[LESGO_P], F_[LESGO_DPDZ], F_[LESGO_RHSZ], F_[LESGO_U], F_[LESGO_V],
-                                                  F_[LESGO_W], kp_);
-    else
-      k_wproj<R, false><<<grid1(n), 256, 0, st_>>>(F_[LESGO_P], F_[LESGO_DPDZ], F_[LESGO_RHSZ], F_[LESGO_U], F_[LESGO_V],
-                                                   F_[LESGO_W], kp_);
+    auto wproj = fused ? k_wproj<R, true> : k_wproj<R, false>;
+    wproj<<<grid1((n + 1) / 2), 256, 0, st_>>>(F_[LESGO_P], F_[LESGO_DPDZ], F_[LESGO_RHSZ], F_[LESGO_U], F_[LESGO_V],
+                                               F_[LESGO_W], kp_);
     post("press.wproj", (fused ? 5.0 : 2.0) * n * sizeof(R));
   }
 
