@@ -12,7 +12,7 @@ template <typename A, class Dst> void rx_inv(const RxGeom<A>& g, const cplx<A>* 
 template <typename A> void rx_fwd21(const RxGeom<A>& g, const SrcLagrange<A>& src, cplx<A>* out, cudaStream_t st);
 template <typename A> void rx_inv42(const RxGeom<A>& g, const cplx<A>* in, const DstLagrange<A>& dst, cudaStream_t st);
 
-enum RyKind { RY_FILT, RY_DIV, RY_PAD, RY_UNPAD, RY_TEST1, RY_TEST2 };
+enum RyKind { RY_FILT, RY_DIV, RY_PAD, RY_VPAD, RY_UNPAD, RY_TEST1, RY_TEST2 };
 // ny rows (the small grid's count) of nf fields, nlev planes
 template <typename A>
 void ry_pass(RyKind kind, const RyArgs<A, cplx<A>, cplx<A>>& a, int ny, int nlev, int nf, cudaStream_t st);

@@ -57,6 +57,7 @@ void ry_pass(RyKind kind, const RyArgs<A, cplx<A>, cplx<A>>& a, int ny, int nlev
       case RY_FILT: go(k_ry_filt<A, R1, R2>, t1, 2 * e + kYC); break;
       case RY_DIV: go(k_ry_div<A, R1, R2>, t1, 2 * e + R2 * kYC); break;
       case RY_PAD: go(k_ry_pad<A, R1, R2>, t2, e + eb); break;
+      case RY_VPAD: go(k_ry_vpad<A, R1, R2>, t2, e + eb); break;
       case RY_UNPAD: go(k_ry_unpad<A, R1, R2>, t2, e + eb); break;
       case RY_TEST1: go(k_ry_test<A, R1, R2, false>, t1, 2 * e); break;
       case RY_TEST2: go(k_ry_test<A, R1, R2, true>, t1, 2 * e); break;

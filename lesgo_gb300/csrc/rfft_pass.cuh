@@ -500,6 +500,12 @@ struct RyArgs {
   const A *kxw, *kyw, *G1, *G2;
   int zero1, zero2;          // first columns past the G1 / G2 cutoffs
   int ia[3], ib[3];          // k_ry_div: the input fields of each output
+  A gs;                      // k_ry_test with one filter: factor of G1
+  // k_ry_vpad: 1/dz, the bottom condition, its velocity, and the wall law's
+  // constants per instance (wall_equilibrium)
+  A inv_dz, ubot, lbc_scale;
+  int lbc;
+  const double* wall_i;
   __device__ __forceinline__ long long plane_in(int li) const {
     const int inst = fnli.div(li), lv = li - inst * nli;
     return (long long)inst * in_inst_levels + in_lev0 + lv * in_levstride;
@@ -680,6 +686,17 @@ __global__ void __launch_bounds__(kYC * cmax(R1, R2)) k_ry_div(RyArgs<A, cplx<A>
   }
 }
 
+// The R2 modes of a thread of ny rows as the 3 R2 / 2 of 3 ny / 2 rows: the
+// upper half moves up, the Nyquist row and the new ones are zero.
+template <typename T2, int R2>
+__device__ __forceinline__ void ry_relabel(T2* v, int t) {
+#pragma unroll
+  for (int j = R2 - 1; j >= R2 / 2; --j) v[j + R2 / 2] = v[j];
+#pragma unroll
+  for (int j = R2 / 2; j < R2; ++j) v[j] = czero<T2>();
+  if (t == 0) v[R2] = czero<T2>();
+}
+
 // 3/2 padding: ny rows -> 3 ny / 2 rows (padd, fft.f90:43-72).
 template <typename A, int R1, int R2>
 __global__ void __launch_bounds__(kYC * cmax(R1, 3 * R2 / 2)) k_ry_pad(RyArgs<A, cplx<A>, cplx<A>> a) {
@@ -689,15 +706,92 @@ __global__ void __launch_bounds__(kYC * cmax(R1, 3 * R2 / 2)) k_ry_pad(RyArgs<A,
   T2 v[cmax(R1, S2)];
   if (t < R2) ry_load<R1>(a.in + f * a.in_fs + pin * N * a.K + t * a.K + kx, R2 * a.K, live, v);
   ry_fwd<T2, R1, R2>(v, W0, a.twn, t, c);
-  if (t < R1) {
-#pragma unroll
-    for (int j = R2 - 1; j >= R2 / 2; --j) v[j + R2 / 2] = v[j];
-#pragma unroll
-    for (int j = R2 / 2; j < R2; ++j) v[j] = czero<T2>();
-    if (t == 0) v[R2] = czero<T2>();   // the Nyquist row
-  }
+  ry_relabel<T2, R2>(v, t);
   ry_inv<T2, R1, S2>(v, W1, a.twm, t, c);
   if (t < S2) ry_store<R1>(a.out + f * a.out_fs + (long long)li * M * a.K + t * a.K + kx, S2 * a.K, live, v);
+}
+
+// 3/2 padding of u, v, w and of the vorticity formed from their modes
+// (convec.f90:71-168): o3 = i kx v - i ky u, and with the staggered
+// differences o1 = i ky w - (v(k) - v(k-1)) / dz, o2 = (u(k) - u(k-1)) / dz -
+// i kx w; at the bottom wall w is averaged over the first two levels and the
+// wall's du/dz, dv/dz are multiples of u, v (less the wall's velocity), so
+// they too stay in the modes.  The inputs are the x spectra of u, v, w alone:
+// the gradients are not transformed again, and the convective term does not
+// wait for them.  (Level nz's o1 and o2 are not used: no product reads them.)
+// blockIdx.z: 0 -> u, w, o2; 1 -> v, o3, o1.
+template <typename A, int R1, int R2>
+__global__ void __launch_bounds__(kYC * cmax(R1, 3 * R2 / 2)) k_ry_vpad(RyArgs<A, cplx<A>, cplx<A>> a) {
+  LESGO_RY_HEAD();
+  constexpr int N = R1 * R2, S2 = 3 * R2 / 2, M = R1 * S2;
+  T2* W1 = W0 + ry_elems<R1, R2>();
+  const int inst = a.fnli.div(li), k = li - inst * a.nli + 1;
+  const bool wall = k == 1;
+  const int step = R2 * a.K;
+  const T2* src = a.in + pin * N * a.K + t * a.K + kx;
+  const long long lev = (long long)N * a.K;
+  T2* dst = a.out + (long long)li * M * a.K + t * a.K + kx;
+  const A kxv = live ? a.kxw[kx] : (A)0;
+  // the wall's gradient over velocity, and the velocity that its mean mode loses
+  const A ws = a.lbc == 2 ? (A)a.wall_i[2 * inst + 1] : a.lbc_scale;
+  const A wu = (wall && a.lbc == 1 && kx == 0 && t == 0) ? a.ubot : (A)0;
+  T2 v[cmax(R1, S2)];
+  auto fwd = [&](int q, int up) {   // modes of field q (0 u, 1 v, 2 w), `up` levels above this one
+    if (t < R2) ry_load<R1>(src + q * a.in_fs + up * lev, step, live, v);
+    ry_fwd<T2, R1, R2>(v, W0, a.twn, t, c);
+  };
+  auto put = [&](int o) {
+    ry_relabel<T2, R2>(v, t);
+    ry_inv<T2, R1, S2>(v, W1, a.twm, t, c);
+    if (t < S2) ry_store<R1>(dst + o * a.out_fs, S2 * a.K, live, v);
+  };
+  // i kxv a + b, and i ky of mode (t, j) times a
+  auto ikx = [&](T2 x) { return mkc(-kxv * x.y, kxv * x.x); };
+  auto iky = [&](T2 x, int j) {
+    const A w = t < R1 ? a.kyw[t + R1 * j] : (A)0;
+    return mkc(-w * x.y, w * x.x);
+  };
+  const A h = FftConst<A>::half();
+  T2 p[R2], r[R2];
+  auto keep = [&](T2* x) {
+#pragma unroll
+    for (int j = 0; j < R2; ++j) x[j] = v[j];
+  };
+  if (f == 0) {
+    fwd(0, 0);
+    keep(p);   // u
+    put(0);
+    fwd(2, 0);
+    keep(r);   // w
+    put(2);
+    fwd(wall ? 2 : 0, wall ? 1 : -1);   // w above, or u below
+#pragma unroll
+    for (int j = 0; j < R2; ++j) {
+      if (!wall) v[j] = csub(cscale(csub(p[j], v[j]), a.inv_dz), ikx(r[j]));
+      else if (a.lbc == 0) v[j] = czero<T2>();
+      else v[j] = csub(cscale(mkc(j == 0 ? p[j].x - wu : p[j].x, p[j].y), ws), ikx(cscale(cadd(r[j], v[j]), h)));
+    }
+    put(4);
+  } else {
+    fwd(1, 0);
+    keep(p);   // v
+    put(1);
+    fwd(0, 0);
+#pragma unroll
+    for (int j = 0; j < R2; ++j) v[j] = csub(ikx(p[j]), iky(v[j], j));
+    put(5);
+    fwd(wall ? 2 : 1, wall ? 1 : -1);   // w above, or v below
+    keep(r);
+    __syncthreads();   // two forward transforms in a row share W0
+    fwd(2, 0);
+#pragma unroll
+    for (int j = 0; j < R2; ++j) {
+      if (!wall) v[j] = csub(iky(v[j], j), cscale(csub(p[j], r[j]), a.inv_dz));
+      else if (a.lbc == 0) v[j] = czero<T2>();
+      else v[j] = csub(iky(cscale(cadd(v[j], r[j]), h), j), cscale(p[j], ws));
+    }
+    put(3);
+  }
 }
 
 // Truncation: 3 ny / 2 rows -> ny rows (unpadd, fft.f90:75-99).
@@ -787,7 +881,10 @@ __global__ void __launch_bounds__(kYC * cmax(R1, R2)) k_ry_test(RyArgs<A, cplx<A
   auto times = [&](const A* G) {
     if (t < R1) {
 #pragma unroll
-      for (int k2 = 0; k2 < R2; ++k2) v[k2] = cscale(x[k2], live ? G[(t + R1 * k2) * a.lh + kx] : (A)0);
+      for (int k2 = 0; k2 < R2; ++k2) {
+        const A w = live ? G[(t + R1 * k2) * a.lh + kx] : (A)0;
+        v[k2] = cscale(x[k2], BOTH ? w : w * a.gs);
+      }
     }
   };
 #pragma unroll

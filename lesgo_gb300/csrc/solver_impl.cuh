@@ -1497,23 +1497,65 @@ class Solver : public SolverBase {
   }
 
   void step_body(bool lag_any) {
-    step_begin_kernels();
     // main.f90:155-172: derivatives (RHS_f is saved inside the fused convec epilogue)
     const InstMap im = imf(d_.nz);
     SrcFields<R, 3> src{{F_[LESGO_U], F_[LESGO_V], F_[LESGO_W]}, (R)(1.0 / ((double)d_.nx * d_.ny)), 1, 1, d_.ld,
                         kp_.plane, im};
+    DstFields<R, 9> dst{{F_[LESGO_U], F_[LESGO_DUDX], F_[LESGO_DUDY], F_[LESGO_V], F_[LESGO_DVDX], F_[LESGO_DVDY],
+                         F_[LESGO_W], F_[LESGO_DWDX], F_[LESGO_DWDY]}, 1, 1, d_.ld, kp_.plane, im};
+    // Where the convective term takes its vorticity from the velocity's modes
+    // (k_ry_vpad), it needs only filt_da's forward x pass.  Branch: the
+    // wall-model inputs (main.f90:180-189) and the convective term, then the
+    // applied forcing (filtered velocity of this step, main.f90:248-257).
+    // Main: the derivatives, sgs_stag with ddz and the wall values fused
+    // (main.f90:164-189), the dynamic update, the stress divergence.  They
+    // meet before the RHS epilogue, which reads all of them.  (The branch
+    // starts behind filt_da's y pass, which reads the spectra that the
+    // convective term's rows write over.)
+    if (vpad_) {
+      if (d_.p.use_cfl_dt) {
+        step_begin_kernels();   // reads the velocity that filt_da replaces
+      } else {
+        fork(7);
+        on_branch([&] { step_begin_kernels(); });
+      }
+      xfwd<3>(src, d_.nx, d_.ny, d_.nz, cvA_, px_, "filt_da.xfwd");
+      y_pass(RY_FILT, cvA_, specB_, d_.nz, 3, "filt_da.ypass");
+      fork(0);
+      on_branch([&] { wall_planes_from_spectra(); });
+      mark(8);
+      on_branch([&] {
+        y_pass(RY_VPAD, cvA_, cvB_, d_.nz, 2, "convec.ypass_vpad");
+        convec_rows_and_back();
+      });
+      xinv<9>(dst, specB_, d_.nx, d_.ny, d_.nz, px_, "filt_da.xinv");
+      if (kp_.turbines) {
+        fork(9);
+        on_branch([&] { turb_impl(); });
+      }
+      if (wall_law()) await(8);
+      if (lag_any) {
+        column<COL_DDZ | COL_STORE_S>();
+        lagrange();
+        column<COL_READ_S | COL_TAU>();
+      } else {
+        column<COL_DDZ | COL_TAU>();
+      }
+      divstress(3);
+      join(2);
+      convec_part2(true);
+      pressure_impl(true);
+      return;
+    }
+    step_begin_kernels();
     // into the convective term's spectra, which reuses them (convec_part1)
     xfwd<3>(src, d_.nx, d_.ny, d_.nz, cvA_, px_, "filt_da.xfwd");
     y_pass(RY_FILT, cvA_, specB_, d_.nz, 3, "filt_da.ypass");
-    DstFields<R, 9> dst{{F_[LESGO_U], F_[LESGO_DUDX], F_[LESGO_DUDY], F_[LESGO_V], F_[LESGO_DVDX], F_[LESGO_DVDY],
-                         F_[LESGO_W], F_[LESGO_DWDX], F_[LESGO_DWDY]}, 1, 1, d_.ld, kp_.plane, im};
     xinv<9>(dst, specB_, d_.nx, d_.ny, d_.nz, px_, "filt_da.xinv");
-    // Two branches from here.  Branch: the applied forcing (filtered velocity
-    // of this step, main.f90:248-257), then, once the column pass is done,
-    // the dynamic update and the stress divergence.  Main: the wall-model
-    // inputs (main.f90:180-189), sgs_stag with ddz and the wall values fused
-    // (main.f90:164-189), the convective term.  They meet before the RHS
-    // epilogue, which reads all of them.
+    // Otherwise the vorticity waits for the column pass.  Branch: the applied
+    // forcing, then, once the column pass is done, the dynamic update and the
+    // stress divergence.  Main: the wall-model inputs, the column pass, the
+    // convective term.
     fork(0);
     if (kp_.turbines) on_branch([&] { turb_impl(); });
     wall_planes();
@@ -1689,6 +1731,9 @@ class Solver : public SolverBase {
     py_ = make_plan(d_.ny);
     pxb_ = make_plan(d_.nx2 / 2);
     pyb_ = make_plan(d_.ny2);
+    // (the tensor-core x transform keeps the vorticity's own forward pass)
+    const char* xd = std::getenv("LESGO_XDFT");
+    const bool xdft = std::is_same<A, float>::value && xd && std::strcmp(xd, "1") == 0;
     if (kRf<A> && rf_) {
       int r1 = 0, r2 = 0;
       if (rx_factors(d_.nx / 2, &r1, &r2)) rx_tw_ = rf_table(r1, r2);
@@ -1696,6 +1741,7 @@ class Solver : public SolverBase {
         ry_twn_ = rf_table(r1, r2);
         ry_twm_ = rf_table(r1, 3 * r2 / 2);
       }
+      vpad_ = rx_tw_ && ry_twn_ && !xdft;
       if (kRfRows<A> && conv_rows_ && rxb_factors(d_.nx2 / 2, &r1, &r2)) rxb_tw_ = rf_table(r1, r2);
     }
     // wavenumbers (fft.f90:130-160) for kx < nx/2 and every ky row
@@ -2005,13 +2051,16 @@ class Solver : public SolverBase {
     a.twn = ry_twn_; a.twm = ry_twm_;
     a.kxw = kxw_; a.kyw = kyw_; a.G1 = G1_; a.G2 = G2_;
     a.zero1 = kmax_g_[0] + 1; a.zero2 = kmax_g_[1] + 1;
+    a.gs = (A)1;
+    a.inv_dz = (A)(1.0 / d_.dz); a.ubot = (A)d_.p.ubot; a.lbc_scale = (A)(1.0 / (0.5 * d_.dz));
+    a.lbc = kp_.lbc; a.wall_i = wall_d_;
     return a;
   }
   // The y passes of the step: transforms in registers where ny is one of
   // their lengths, else the run-time radix stages.
   void y_pass(RyKind kind, const T2* in, T2* out, int nli, int nf, const char* tag) {
     const int ny = d_.ny, ny2 = d_.ny2;
-    const int rin = kind == RY_UNPAD ? ny2 : ny, rout = kind == RY_PAD ? ny2 : ny;
+    const int rin = kind == RY_UNPAD ? ny2 : ny, rout = kind == RY_PAD || kind == RY_VPAD ? ny2 : ny;
     if constexpr (kRf<A>) {
       if (ry_twn_) {
         const int nlev = nli * kp_.ninst;
@@ -2022,7 +2071,8 @@ class Solver : public SolverBase {
         ry_pass<A>(kind, a, ny, nlev, nf, st_);
         const int no = kind == RY_FILT ? 3 : kind == RY_TEST2 ? 2 : 1;
         const double ni = kind == RY_DIV ? (nf == 3 ? 5.0 / 3.0 : nf == 2 ? 1.5 : 2.0) : 1.0;
-        post(tag, (double)nf * nlev * d_.K * (ni * rin + no * rout) * sizeof(T2));
+        const double units = kind == RY_VPAD ? 3.0 * rin + 6.0 * rout : nf * (ni * rin + no * rout);
+        post(tag, units * nlev * d_.K * sizeof(T2));
         return;
       }
     }
@@ -2042,6 +2092,8 @@ class Solver : public SolverBase {
       case RY_PAD:
         ypass_lin<1, 1, true, true, T2, T2>(in, 0, 1, nli, ny, out, ny2, nli, nf, ROW_PAD, {{MUL_ONE}}, tag);
         break;
+      case RY_VPAD:
+        throw Error(LESGO_ERR_UNSUPPORTED, "vorticity from the velocity's modes: length");
       case RY_UNPAD:
         ypass_lin<1, 1, true, true, T2, T2>(in, 0, 1, nli, ny2, out, ny, nli, nf, ROW_UNPAD, {{MUL_ONE}}, tag);
         break;
@@ -2100,6 +2152,24 @@ class Solver : public SolverBase {
     } else {
       DstFields<R, 2> dst{{oa, ob}, 0, 1, d_.ld, 0, InstMap(1, ostr)};
       xinv<2>(dst, outp, d_.nx, d_.ny, 1, px_, "wall_filter.xinv");
+    }
+  }
+  // The same planes of u and v from their x spectra (filt_da's forward pass,
+  // which scales by 1/(nx ny): G1's own factor is taken out again).  The
+  // filters drop the modes that filt_da drops, so the spectra before it serve.
+  bool wall_law() const { return d_.p.lbc_mom == 2 || d_.p.ubc_mom == 2; }
+  void wall_planes_from_spectra() {
+    if constexpr (kRf<A>) {
+      for (int top = 0; top < 2; ++top) {
+        if ((top ? d_.p.ubc_mom : d_.p.lbc_mom) != 2) continue;
+        RyArgs<A, T2, T2> a = ry_args(cvA_, top ? d_.nz - 2 : 0, 1, d_.nz, d_.ny, specC_, d_.ny, 1);
+        a.gs = (A)((double)d_.nx * d_.ny);
+        pre();
+        ry_pass<A>(RY_TEST1, a, d_.ny, kp_.ninst, 2, st_);
+        post("wall_filter.ypass", 4.0 * kp_.ninst * d_.K * d_.ny * sizeof(T2));
+        DstFields<R, 2> dst{{wall_[2 * top], wall_[2 * top + 1]}, 0, 1, d_.ld, 0, InstMap(1, kp_.plane)};
+        xinv<2>(dst, specC_, d_.nx, d_.ny, 1, px_, "wall_filter.xinv");
+      }
     }
   }
   void wall_planes() {
@@ -2183,7 +2253,6 @@ class Solver : public SolverBase {
   void convec_part1(bool uvw_ready) {
     const R c = (R)(1.0 / ((double)d_.nx * d_.ny));
     const InstMap im = imf(d_.nz);
-    const InstMap imb(d_.nz, kp_.istride_big);
     if (uvw_ready) {
       SrcVort<R, true> sv{F_[LESGO_U], F_[LESGO_V], F_[LESGO_W], F_[LESGO_DUDY], F_[LESGO_DUDZ], F_[LESGO_DVDX],
                           F_[LESGO_DVDZ], F_[LESGO_DWDX], F_[LESGO_DWDY], c, d_.ld, d_.nz, kp_.lbc, kp_.ubc,
@@ -2195,6 +2264,12 @@ class Solver : public SolverBase {
       xfwd<6>(sv, d_.nx, d_.ny, d_.nz, cvA_, px_, "convec.xfwd", 9);
     }
     y_pass(RY_PAD, cvA_, cvB_, d_.nz, 6, "convec.ypass_pad");
+    convec_rows_and_back();
+  }
+  // From the six padded spectra of cvB_ to the three products' spectra on the
+  // small grid, in cvB_ again.
+  void convec_rows_and_back() {
+    const InstMap imb(d_.nz, kp_.istride_big);
     if (conv_rows_) {
       convec_rows(HostCvt<A>::from(1.0L / ((long double)d_.nx2 * d_.ny2)));
     } else {
@@ -2303,6 +2378,14 @@ class Solver : public SolverBase {
     if (serial()) return;
     CK(cudaEventRecord(ev_[e], st2_));
     CK(cudaStreamWaitEvent(st_, ev_[e], 0));
+  }
+  // A point of the branch (mark) that the main stream waits for (await)
+  // without the rest of the branch.
+  void mark(int e) {
+    if (!serial()) CK(cudaEventRecord(ev_[e], st2_));
+  }
+  void await(int e) {
+    if (!serial()) CK(cudaStreamWaitEvent(st_, ev_[e], 0));
   }
   template <class F>
   void on_branch(F&& fn) {
@@ -2426,7 +2509,7 @@ class Solver : public SolverBase {
   double* sc_d_ = nullptr;                   // step constants [cap][SC_N]
   T2 *cvA_ = nullptr, *cvB_ = nullptr;       // convective-term spectra
   cudaStream_t st2_ = nullptr;               // second branch of the fused step
-  cudaEvent_t ev_[8] = {};
+  cudaEvent_t ev_[10] = {};
   static constexpr int kRing = 64;
   int* ring_h_ = nullptr;                    // pinned [kRing][cap]
   cudaEvent_t ring_ev_[kRing] = {};
@@ -2454,6 +2537,7 @@ class Solver : public SolverBase {
   // twiddles of the register transforms (null: the length is not one of
   // theirs): x rows, y columns of ny and 3 ny / 2, 3/2-grid x rows
   bool rf_ = true;
+  bool vpad_ = false;              // the fused step's vorticity from the velocity's modes
   T2 *rx_tw_ = nullptr, *ry_twn_ = nullptr, *ry_twm_ = nullptr, *rxb_tw_ = nullptr;
   A *kxw_ = nullptr, *kyw_ = nullptr, *G1_ = nullptr, *G2_ = nullptr;
   int kmax_g_[2] = {1 << 30, 1 << 30};   // largest kx column with a nonzero G1 / G2 weight
