@@ -23,6 +23,7 @@
 #include <type_traits>
 
 #include "df64.cuh"
+#include "fp64_light.cuh"
 
 namespace lesgo {
 

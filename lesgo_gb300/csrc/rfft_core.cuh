@@ -154,20 +154,4 @@ template <int A, int B> struct Len {
   static constexpr int R1 = A, R2 = B, N = A * B;
 };
 
-// FP32 <-> FP64 without the FP64 pipe, on which a conversion costs as much
-// as an addition: exponent and mantissa are moved with integer operations.
-// `odd` collects whether a value needs the instruction (zeros, subnormals,
-// infinities, NaN; for narrow_fast also results outside the normal range).
-__device__ __forceinline__ double widen_fast(float x, bool& odd) {
-  const unsigned b = __float_as_uint(x);
-  odd |= (b & 0x7f800000u) - 0x00800000u >= 0x7f000000u;   // exponent 0 or 255
-  return __hiloint2double((int)(((b & 0x7fffffffu) >> 3) + 0x38000000u | (b & 0x80000000u)), (int)(b << 29));
-}
-__device__ __forceinline__ float narrow_fast(double x, bool& odd) {   // round to nearest even
-  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
-  odd |= (hi & 0x7fffffffu) - 0x38100000u >= 0x0fd00000u;   // outside 2^-126 .. 2^127
-  const unsigned l = lo + 0x0fffffffu + ((lo >> 29) & 1u), h = (hi & 0x7fffffffu) + (l < lo ? 1u : 0u);
-  return __uint_as_float((__funnelshift_l(l, h, 3) - 0xc0000000u) | (hi & 0x80000000u));
-}
-
 }  // namespace lesgo

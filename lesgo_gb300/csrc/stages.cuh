@@ -428,13 +428,6 @@ struct DstPress {
   }
 };
 
-// x^(-1/8) for x > 0 (the Lagrangian time scale, lagrange_Sdep.f90's
-// Tn**(-1/8)): two square roots and a reciprocal square root, within a few
-// ulps of pow and far cheaper than pow in FP64, where these three powers
-// per point had bound the whole Lagrangian epilogue.
-__device__ __forceinline__ double inv_root8(double x) { return rsqrt(sqrt(sqrt(x))); }
-__device__ __forceinline__ float inv_root8(float x) { return rsqrtf(sqrtf(sqrtf(x))); }
-
 // lagrange_Sdep.f90:110-404 pointwise part: Leonard terms L, Q, model
 // tensors M, N, their contractions, the Lagrangian relaxation of F_LM,
 // F_MM, F_QN, F_NN, beta and Cs^2.  vals[2q] = quantity q at 2 Delta,
@@ -491,29 +484,29 @@ struct DstLagrange {
     Tn = (R)opftdelta * inv_root8(Tn);
     Tn = max(zero, Tn);
     const R ldt = (R)sc[inst * SC_N + SC_LDT];
-    R dumfac = ldt / Tn;
-    R epsi = dumfac / ((R)1 + dumfac);
+    // epsi = (ldt/Tn) / (1 + ldt/Tn)
+    R epsi = div_light(ldt, Tn + ldt);
     fLM = epsi * LM + ((R)1 - epsi) * fLM;
     fMM = epsi * MM + ((R)1 - epsi) * fMM;
     fLM = max(zero, fLM);
-    R cs2d = fLM / (fMM + zero);
+    R cs2d = div_light(fLM, fMM + zero);
     cs2d = max(zero, cs2d);
     if (init_qn) { fNN = NN; fQN = (R)0.03 * NN; }
     Tn = max(fQN * fNN, zero);
     Tn = (R)opftdelta * inv_root8(Tn);
     Tn = max(zero, Tn);
-    dumfac = ldt / Tn;
-    epsi = dumfac / ((R)1 + dumfac);
+    epsi = div_light(ldt, Tn + ldt);
     fQN = epsi * QN + ((R)1 - epsi) * fQN;
     fNN = epsi * NN + ((R)1 - epsi) * fNN;
     fQN = max(zero, fQN);
-    R cs4d = fQN / (fNN + zero);
+    R cs4d = div_light(fQN, fNN + zero);
     cs4d = max(zero, cs4d);
-    R beta = beta_exp_one ? cs4d / cs2d : pow(cs4d / cs2d, (R)beta_exp);
+    const R ratio = div_light(cs4d, cs2d);
+    R beta = beta_exp_one ? ratio : pow(ratio, (R)beta_exp);
     if (k == nz && ubc == 0) beta = (R)1;
     if (k == 1 && lbc == 0) beta = (R)1;
     const R betaclip = max(beta, (R)1 / (tf1 * tf2));
-    const R csn = max(zero, cs2d / betaclip);
+    const R csn = max(zero, div_light(cs2d, betaclip));
     FLM[q] = (R)fLM; FMM[q] = (R)fMM; FQN[q] = (R)fQN; FNN[q] = (R)fNN;
     Cs[q] = csn;
     Beta[q] = beta;
