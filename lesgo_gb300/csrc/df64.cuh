@@ -25,7 +25,7 @@
 
 namespace lesgo {
 
-struct df64 {
+struct alignas(8) df64 {
   float hi, lo;
 };
 

