@@ -16,7 +16,8 @@ LIB = os.path.join(HERE, "liblesgo_gpu.so")
 OBJDIR = os.path.join(HERE, "_build")
 SOURCES = [os.path.join(CSRC, f) for f in (
     "solver.cu", "solver_fp32.cu", "solver_fp64.cu", "solver_dw.cu", "rfft_xf32.cu", "rfft_xi32.cu", "rfft_y32.cu",
-    "rfft_rows32.cu", "rfft_xf64.cu", "rfft_xi64.cu", "rfft_y64.cu")]
+    "rfft_rows32.cu", "rfft_xf64.cu", "rfft_xi64.cu", "rfft_y64.cu",
+    "rfft_ydw_filt.cu", "rfft_ydw_div.cu", "rfft_ydw_pad.cu", "rfft_ydw_unpad.cu")]
 DEPS = SOURCES + sorted(os.path.join(CSRC, f) for f in os.listdir(CSRC)
                         if f.endswith((".cuh", ".hpp"))) + [os.path.join(ROOT, "include", "lesgo_gpu.h")]
 

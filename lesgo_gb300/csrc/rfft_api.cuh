@@ -13,9 +13,18 @@ template <typename A> void rx_fwd21(const RxGeom<A>& g, const SrcLagrange<A>& sr
 template <typename A> void rx_inv42(const RxGeom<A>& g, const cplx<A>* in, const DstLagrange<A>& dst, cudaStream_t st);
 
 enum RyKind { RY_FILT, RY_DIV, RY_PAD, RY_VPAD, RY_UNPAD, RY_TEST1, RY_TEST2 };
+// The double-word form has the four kinds that gain by it (128^3, us against
+// the run-time radix stages): filt_da 93 (150), divergence 107 (191), pad 161
+// (226), unpad 91 (114).  With two filters, the forward modes kept for both,
+// registers leave too few warps (852 against 624), the pressure's passes
+// gain nothing (55 against 59, 53 against 51), and RY_VPAD's code alone would
+// be several hundred KB.
+template <typename A> constexpr bool kRyKind(RyKind k) {
+  return !std::is_same<A, df64>::value || k == RY_FILT || k == RY_DIV || k == RY_PAD || k == RY_UNPAD;
+}
 // ny rows (the small grid's count) of nf fields, nlev planes
-template <typename A>
-void ry_pass(RyKind kind, const RyArgs<A, cplx<A>, cplx<A>>& a, int ny, int nlev, int nf, cudaStream_t st);
+template <typename A, RyKind KIND>
+void ry_pass(const RyArgs<A, cplx<A>, cplx<A>>& a, int ny, int nlev, int nf, cudaStream_t st);
 template <typename A>
 void ry_spec(const RyArgs<A, cplx<A>, double2>& a, int ny, int nlev, int nf, cudaStream_t st);
 template <typename A>

@@ -35,6 +35,12 @@ __host__ __device__ constexpr double root_sin(int m, int R) {
   return root_cos((t + 108) % 144, 144);
 }
 
+// a table value in the arithmetic A (double-word: hi and the rounded rest)
+template <typename A> __host__ __device__ constexpr A root_const(double v) {
+  if constexpr (std::is_same<A, df64>::value) return df64{(float)v, (float)(v - (double)(float)v)};
+  else return (A)v;
+}
+
 // a * exp(-2 pi i M / R), or its conjugate rotation with INV
 template <int M, int R, bool INV, typename T2>
 __device__ __forceinline__ T2 mul_root(T2 a) {
@@ -45,14 +51,17 @@ __device__ __forceinline__ T2 mul_root(T2 a) {
   else if constexpr (2 * m == R) return mkc(-a.x, -a.y);
   else if constexpr (4 * m == 3 * R) return INV ? mul_mi(a) : mul_pi(a);
   else if constexpr (8 * m == R || 8 * m == 3 * R || 8 * m == 5 * R || 8 * m == 7 * R) {
-    constexpr A c = (A)root_cos(m, R);   // +- sqrt(1/2)
-    constexpr A s = (A)(INV ? root_sin(m, R) : -root_sin(m, R));
-    if constexpr ((c > 0) == (s > 0)) return mkc(c * (a.x - a.y), c * (a.x + a.y));
+    constexpr double cd = root_cos(m, R), sd = INV ? root_sin(m, R) : -root_sin(m, R);
+    constexpr A c = root_const<A>(cd);   // +- sqrt(1/2)
+    if constexpr (std::is_same<T2, dfc>::value)
+      return cscale((cd > 0) == (sd > 0) ? csub(a, mul_mi(a)) : cadd(a, mul_mi(a)), c);
+    else if constexpr ((cd > 0) == (sd > 0)) return mkc(c * (a.x - a.y), c * (a.x + a.y));
     else return mkc(c * (a.x + a.y), c * (a.y - a.x));
   } else {
-    constexpr A c = (A)root_cos(m, R);
-    constexpr A s = (A)(INV ? root_sin(m, R) : -root_sin(m, R));
-    return mkc(a.x * c - a.y * s, a.x * s + a.y * c);
+    constexpr A c = root_const<A>(root_cos(m, R));
+    constexpr A s = root_const<A>(INV ? root_sin(m, R) : -root_sin(m, R));
+    if constexpr (std::is_same<T2, dfc>::value) return cmul(a, mkc(c, s));
+    else return mkc(a.x * c - a.y * s, a.x * s + a.y * c);
   }
 }
 
@@ -146,6 +155,16 @@ __host__ __device__ constexpr int odd_up(int a) { return a | 1; }
 template <bool INV, typename T2> __device__ __forceinline__ T2 mul_tw(T2 a, const T2* w) {
   const T2 t = ldt(w);
   return INV ? cmulconj(a, t) : cmul(a, t);
+}
+
+// i k a, and a + i k b
+template <typename T2, typename A> __device__ __forceinline__ T2 mul_ik(A k, T2 a) {
+  if constexpr (std::is_same<T2, dfc>::value) return cscale(mul_pi(a), k);
+  else return mkc(-k * a.y, k * a.x);
+}
+template <typename T2, typename A> __device__ __forceinline__ T2 add_ik(T2 a, A k, T2 b) {
+  if constexpr (std::is_same<T2, dfc>::value) return cadd(a, mul_ik(k, b));
+  else return mkc(a.x - k * b.y, a.y + k * b.x);
 }
 
 // The factors of a length, chosen at compile time from a list; the host

@@ -42,8 +42,8 @@ template <typename A> void rx_inv42(const RxGeom<A>& g, const cplx<A>* in, const
   });
 }
 
-template <typename A>
-void ry_pass(RyKind kind, const RyArgs<A, cplx<A>, cplx<A>>& a, int ny, int nlev, int nf, cudaStream_t st) {
+template <typename A, RyKind KIND>
+void ry_pass(const RyArgs<A, cplx<A>, cplx<A>>& a, int ny, int nlev, int nf, cudaStream_t st) {
   with_ry(ny, [&](auto len) {
     constexpr int R1 = decltype(len)::R1, R2 = decltype(len)::R2, S2 = 3 * R2 / 2;
     constexpr size_t e = ry_elems<R1, R2>(), eb = ry_elems<R1, S2>();
@@ -53,15 +53,13 @@ void ry_pass(RyKind kind, const RyArgs<A, cplx<A>, cplx<A>>& a, int ny, int nlev
       kern<<<grid, threads, elems * sizeof(cplx<A>), st>>>(a);
     };
     constexpr int t1 = kYC * cmax(R1, R2), t2 = kYC * cmax(R1, S2);
-    switch (kind) {
-      case RY_FILT: go(k_ry_filt<A, R1, R2>, t1, 2 * e + kYC); break;
-      case RY_DIV: go(k_ry_div<A, R1, R2>, t1, 2 * e + R2 * kYC); break;
-      case RY_PAD: go(k_ry_pad<A, R1, R2>, t2, e + eb); break;
-      case RY_VPAD: go(k_ry_vpad<A, R1, R2>, t2, e + eb); break;
-      case RY_UNPAD: go(k_ry_unpad<A, R1, R2>, t2, e + eb); break;
-      case RY_TEST1: go(k_ry_test<A, R1, R2, false>, t1, 2 * e); break;
-      case RY_TEST2: go(k_ry_test<A, R1, R2, true>, t1, 2 * e); break;
-    }
+    if constexpr (KIND == RY_FILT) go(k_ry_filt<A, R1, R2>, t1, 2 * e + kYC);
+    if constexpr (KIND == RY_DIV) go(k_ry_div<A, R1, R2>, t1, 2 * e + R2 * kYC);
+    if constexpr (KIND == RY_PAD) go(k_ry_pad<A, R1, R2>, t2, e + eb);
+    if constexpr (KIND == RY_VPAD) go(k_ry_vpad<A, R1, R2>, t2, e + eb);
+    if constexpr (KIND == RY_UNPAD) go(k_ry_unpad<A, R1, R2>, t2, e + eb);
+    if constexpr (KIND == RY_TEST1) go(k_ry_test<A, R1, R2, false>, t1, 2 * e);
+    if constexpr (KIND == RY_TEST2) go(k_ry_test<A, R1, R2, true>, t1, 2 * e);
   });
 }
 template <typename A>

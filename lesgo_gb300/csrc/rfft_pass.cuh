@@ -598,10 +598,7 @@ template <typename A, int R1, int R2>
 __device__ __forceinline__ void ry_iky(const A* kyw, int t, cplx<A>* v) {
   if (t < R1) {
 #pragma unroll
-    for (int k2 = 0; k2 < R2; ++k2) {
-      const A k = kyw[t + R1 * k2];
-      v[k2] = mkc(-k * v[k2].y, k * v[k2].x);
-    }
+    for (int k2 = 0; k2 < R2; ++k2) v[k2] = mul_ik(kyw[t + R1 * k2], v[k2]);
   }
 }
 
@@ -635,13 +632,13 @@ __global__ void __launch_bounds__(kYC * cmax(R1, R2)) k_ry_filt(RyArgs<A, cplx<A
     T2* d = a.out + (3 * f) * a.out_fs + (long long)li * N * a.K + t * a.K + kx;
     ry_store<R1>(d + 2 * a.out_fs, R2 * a.K, true, v);
     const T2 s = (t & 1) ? mkc(-ny[c].x, -ny[c].y) : ny[c];
-    const A k = a.kxw[kx], n = (A)N;
+    const A k = a.kxw[kx], n = cvt<A>((float)N);
     ry_load<R1>(src, R2 * a.K, true, v);
 #pragma unroll
     for (int j = 0; j < R1; ++j) {
       const T2 x = csub(cscale(v[j], n), s);
       d[j * R2 * a.K] = x;
-      d[a.out_fs + j * R2 * a.K] = mkc(-k * x.y, k * x.x);
+      d[a.out_fs + j * R2 * a.K] = mul_ik(k, x);
     }
   }
 }
@@ -674,14 +671,14 @@ __global__ void __launch_bounds__(kYC * cmax(R1, R2)) k_ry_div(RyArgs<A, cplx<A>
 #pragma unroll
     for (int j = 1; j < R2; ++j) s = cadd(s, sum[j * kYC + c]);
     if (t & 1) s = mkc(-s.x, -s.y);
-    const A k = a.kxw[kx], n = (A)N;
+    const A k = a.kxw[kx], n = cvt<A>((float)N);
     T2* d = a.out + f * a.out_fs + (long long)li * N * a.K + t * a.K + kx;
     T2 x[R1];
     ry_load<R1>(pp, R2 * a.K, true, x);
 #pragma unroll
     for (int j = 0; j < R1; ++j) {
       const T2 y = csub(cscale(x[j], n), s);
-      d[j * R2 * a.K] = mkc(v[j].x - k * y.y, v[j].y + k * y.x);
+      d[j * R2 * a.K] = add_ik(v[j], k, y);
     }
   }
 }
@@ -844,7 +841,7 @@ __global__ void __launch_bounds__(kYC * cmax(R1, R2)) k_ry_phys(RyArgs<A, double
     if constexpr (GRAD) {
       const A k = a.kxw[kx];
 #pragma unroll
-      for (int j = 0; j < R1; ++j) d[a.out_fs + j * R2 * a.K] = mkc(-k * v[j].y, k * v[j].x);
+      for (int j = 0; j < R1; ++j) d[a.out_fs + j * R2 * a.K] = mul_ik(k, v[j]);
     }
   }
   if constexpr (GRAD) {
@@ -882,7 +879,7 @@ __global__ void __launch_bounds__(kYC * cmax(R1, R2)) k_ry_test(RyArgs<A, cplx<A
     if (t < R1) {
 #pragma unroll
       for (int k2 = 0; k2 < R2; ++k2) {
-        const A w = live ? G[(t + R1 * k2) * a.lh + kx] : (A)0;
+        const A w = live ? G[(t + R1 * k2) * a.lh + kx] : FftConst<A>::zero();
         v[k2] = cscale(x[k2], BOTH ? w : w * a.gs);
       }
     }

@@ -1,7 +1,9 @@
 // y passes, double transforms.
 #include "rfft_launch.cuh"
 namespace lesgo {
-template void ry_pass(RyKind, const RyArgs<double, cplx<double>, cplx<double>>&, int, int, int, cudaStream_t);
+#define X(k) template void ry_pass<double, k>(const RyArgs<double, cplx<double>, cplx<double>>&, int, int, int, cudaStream_t);
+X(RY_FILT) X(RY_DIV) X(RY_PAD) X(RY_VPAD) X(RY_UNPAD) X(RY_TEST1) X(RY_TEST2)
+#undef X
 template void ry_spec(const RyArgs<double, cplx<double>, double2>&, int, int, int, cudaStream_t);
 template void ry_phys(bool, const RyArgs<double, double2, cplx<double>>&, int, int, cudaStream_t);
 }  // namespace lesgo

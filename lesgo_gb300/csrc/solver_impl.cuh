@@ -227,6 +227,7 @@ template <> struct HostCvt<df64> {
 
 // Which arithmetic, row loaders and row epilogues have passes with the
 // transforms in registers (rfft_api.cuh).
+// (the double-word form has some of the y passes only: kRyKind)
 template <typename A> constexpr bool kRf = std::is_same<A, float>::value || std::is_same<A, double>::value;
 template <typename A> constexpr bool kRfRows = std::is_same<A, float>::value;
 template <class S> constexpr bool kRxSrc = false;
@@ -1734,9 +1735,9 @@ class Solver : public SolverBase {
     // (the tensor-core x transform keeps the vorticity's own forward pass)
     const char* xd = std::getenv("LESGO_XDFT");
     const bool xdft = std::is_same<A, float>::value && xd && std::strcmp(xd, "1") == 0;
-    if (kRf<A> && rf_) {
+    if (rf_) {
       int r1 = 0, r2 = 0;
-      if (rx_factors(d_.nx / 2, &r1, &r2)) rx_tw_ = rf_table(r1, r2);
+      if (kRf<A> && rx_factors(d_.nx / 2, &r1, &r2)) rx_tw_ = rf_table(r1, r2);
       if (yshort_ && ry_factors(d_.ny, &r1, &r2)) {
         ry_twn_ = rf_table(r1, r2);
         ry_twm_ = rf_table(r1, 3 * r2 / 2);
@@ -2051,8 +2052,9 @@ class Solver : public SolverBase {
     a.twn = ry_twn_; a.twm = ry_twm_;
     a.kxw = kxw_; a.kyw = kyw_; a.G1 = G1_; a.G2 = G2_;
     a.zero1 = kmax_g_[0] + 1; a.zero2 = kmax_g_[1] + 1;
-    a.gs = (A)1;
-    a.inv_dz = (A)(1.0 / d_.dz); a.ubot = (A)d_.p.ubot; a.lbc_scale = (A)(1.0 / (0.5 * d_.dz));
+    a.gs = HostCvt<A>::from(1.0L);
+    a.inv_dz = HostCvt<A>::from(1.0 / d_.dz); a.ubot = HostCvt<A>::from(d_.p.ubot);
+    a.lbc_scale = HostCvt<A>::from(1.0 / (0.5 * d_.dz));
     a.lbc = kp_.lbc; a.wall_i = wall_d_;
     return a;
   }
@@ -2061,20 +2063,31 @@ class Solver : public SolverBase {
   void y_pass(RyKind kind, const T2* in, T2* out, int nli, int nf, const char* tag) {
     const int ny = d_.ny, ny2 = d_.ny2;
     const int rin = kind == RY_UNPAD ? ny2 : ny, rout = kind == RY_PAD || kind == RY_VPAD ? ny2 : ny;
-    if constexpr (kRf<A>) {
-      if (ry_twn_) {
+    auto go = [&](auto kc) {
+      constexpr RyKind k = decltype(kc)::value;
+      if constexpr (kRyKind<A>(k)) {
         const int nlev = nli * kp_.ninst;
         RyArgs<A, T2, T2> a = ry_args(in, 0, 1, nli, rin, out, rout, nli);
         const int ia[3] = {0, 1, 3}, ib[3] = {1, 2, 4};
         for (int i = 0; i < 3; ++i) { a.ia[i] = ia[i]; a.ib[i] = ib[i]; }
         pre();
-        ry_pass<A>(kind, a, ny, nlev, nf, st_);
-        const int no = kind == RY_FILT ? 3 : kind == RY_TEST2 ? 2 : 1;
-        const double ni = kind == RY_DIV ? (nf == 3 ? 5.0 / 3.0 : nf == 2 ? 1.5 : 2.0) : 1.0;
-        const double units = kind == RY_VPAD ? 3.0 * rin + 6.0 * rout : nf * (ni * rin + no * rout);
+        ry_pass<A, k>(a, ny, nlev, nf, st_);
+        const int no = k == RY_FILT ? 3 : k == RY_TEST2 ? 2 : 1;
+        const double ni = k == RY_DIV ? (nf == 3 ? 5.0 / 3.0 : nf == 2 ? 1.5 : 2.0) : 1.0;
+        const double units = k == RY_VPAD ? 3.0 * rin + 6.0 * rout : nf * (ni * rin + no * rout);
         post(tag, units * nlev * d_.K * sizeof(T2));
-        return;
+        return true;
       }
+      return false;
+    };
+    if (ry_twn_) {
+      bool done = false;
+      switch (kind) {
+#define X(k) case k: done = go(std::integral_constant<RyKind, k>{}); break;
+        X(RY_FILT) X(RY_DIV) X(RY_PAD) X(RY_VPAD) X(RY_UNPAD) X(RY_TEST1) X(RY_TEST2)
+#undef X
+      }
+      if (done) return;
     }
     switch (kind) {
       case RY_FILT:
@@ -2165,7 +2178,7 @@ class Solver : public SolverBase {
         RyArgs<A, T2, T2> a = ry_args(cvA_, top ? d_.nz - 2 : 0, 1, d_.nz, d_.ny, specC_, d_.ny, 1);
         a.gs = (A)((double)d_.nx * d_.ny);
         pre();
-        ry_pass<A>(RY_TEST1, a, d_.ny, kp_.ninst, 2, st_);
+        ry_pass<A, RY_TEST1>(a, d_.ny, kp_.ninst, 2, st_);
         post("wall_filter.ypass", 4.0 * kp_.ninst * d_.K * d_.ny * sizeof(T2));
         DstFields<R, 2> dst{{wall_[2 * top], wall_[2 * top + 1]}, 0, 1, d_.ld, 0, InstMap(1, kp_.plane)};
         xinv<2>(dst, specC_, d_.nx, d_.ny, 1, px_, "wall_filter.xinv");

@@ -90,3 +90,27 @@ def test_fp64_steps_match_oracle_and_radix(built_lib, monkeypatch, grid):
         assert e < 1e-11, (f, e)
     g.close()
     r.close()
+
+
+@pytest.mark.parametrize("grid", GRIDS, ids=IDS)
+def test_double_word_steps_match_oracle_and_radix(built_lib, monkeypatch, grid):
+    """The y passes that the double-word form has: 1e-10 against the oracle,
+    and 1e-11 against the run-time radix passes (transforms whose operations
+    round at 2^-46 or so, 1.4e-14, a few tens of them in a chain)."""
+    nx, ny, nz, kw = grid
+    kw = dict(nx=nx, ny=ny, Nz=nz, dt=1e-4, dyn_init=3, cs_count=3, **kw)
+    p, o, g = make_pair(precision="fp64dw", **kw)
+    monkeypatch.setenv("LESGO_RFFT", "0")
+    _, _, r = make_pair(precision="fp64dw", **kw)
+    for _ in range(4):
+        o.step()
+    for h in (g, r):
+        h.step(4)
+        h.sync()
+    for f in ("u", "v", "w", "p"):
+        e = rel_err(p, f, g.get(f), oracle_field(o, f))
+        assert e < 1e-10, (f, e)
+        e = rel_err(p, f, g.get(f), r.get(f))
+        assert e < 1e-11, (f, e)
+    g.close()
+    r.close()
