@@ -9,13 +9,15 @@
 // bandwidth):
 //   filt_da      x 14.3 (20.5; 7.5), y 22.9 (45.6; 15), x inverse 37 (50; 22)
 //   divstress    x 19.8 (30.8; 12.5), y 20.0 (55.4; 10), x inverse 18.6 (36; 11)
-//   convec       x 21.3 (36.3; 11), y pad 35.6 (69.8; 19), y unpad 19.3 (37; 9),
-//                x inverse with AB2 38.0 (43.3; 26)
-//   pressure     x 14.5 (20.9; 7.5), y 18.6 (27.5; 11), y inverse 14.1 (22.6; 6),
+//   convec       y pad with the vorticity 34.5 (x 36.3 and y 69.8; 15),
+//                y unpad 19 (37; 9), x inverse with AB2 38.5 (43.3; 26)
+//   pressure     x 14.5 (20.9; 7.5), y 17.1 (27.5; 11), y inverse 14.1 (22.6; 6),
 //                x inverse with projection 28.5 (31.3; 15)
 //   Lagrangian   x 86 (131; 38), y 84 (244; 79), x inverse 144 (303; 69)
 // and one 48^3 instance 5.0 against 6.6 us for a pass of one wave: the
-// stages' barriers (one per radix stage) were its latency.
+// stages' barriers (one per radix stage) were its latency.  In FP64, which
+// the FP64 pipe bounds: 128^3 37.8 -> 33.2 ms for five steps, 32^3 3.9 -> 3.05
+// ms for ten.
 #pragma once
 #include "rfft_core.cuh"
 #include "stages.cuh"
@@ -717,6 +719,9 @@ __global__ void __launch_bounds__(kYC * cmax(R1, 3 * R2 / 2)) k_ry_pad(RyArgs<A,
 // the gradients are not transformed again, and the convective term does not
 // wait for them.  (Level nz's o1 and o2 are not used: no product reads them.)
 // blockIdx.z: 0 -> u, w, o2; 1 -> v, o3, o1.
+// 34.5 us at 128^3 in the mixed form (unique bytes 15) against 21 for the
+// vorticity's own forward x pass and 35.6 for the padding of six spectra; the
+// step, which no longer waits for the column sweep here, 507 -> 469 us.
 template <typename A, int R1, int R2>
 __global__ void __launch_bounds__(kYC * cmax(R1, 3 * R2 / 2)) k_ry_vpad(RyArgs<A, cplx<A>, cplx<A>> a) {
   LESGO_RY_HEAD();
