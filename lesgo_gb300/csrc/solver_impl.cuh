@@ -1534,7 +1534,9 @@ class Solver : public SolverBase {
         fork(9);
         on_branch([&] { turb_impl(); });
       }
-      if (wall_law()) await(8);
+      // the filtered wall planes, and the step constants that the dynamic
+      // update reads
+      if (wall_law() || lag_any) await(8);
       if (lag_any) {
         column<COL_DDZ | COL_STORE_S>();
         lagrange();
