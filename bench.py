@@ -7,7 +7,7 @@ Lz=1; z0 log-uniform in [1e-5, 1e-3]; own seeded log-law + noise IC;
 Lagrangian scale-dependent SGS updated every 5 steps; dt=2e-4) in the mixed
 form (FP32 bulk, FP64 pressure solve): one batch handle per grid class, every
 kernel advancing the whole class in one launch, graph-replayed steps,
-autotuned tiles, the classes overlapping on their own streams.  The timed
+the classes overlapping on their own streams.  The timed
 region is the steady state (the number of timed steps is rounded up to a
 multiple of 5, the phase of the SGS update).
 
@@ -217,7 +217,7 @@ ONLY_CLASS = None
 
 def make_batches(precision="mixed", split=1):
     """Batch handles of the 48-instance ensemble, every instance added, tile
-    shapes autotuned: one per grid class, or `split` per class (the class's
+    shapes autotuned where a pass has them: one per grid class, or `split` per class (the class's
     instances dealt in turn)."""
     from lesgo_gb300.solver import LesgoBatch
     by_grid = {}
@@ -278,7 +278,7 @@ def merge_profiles(reps):
 def time_batched(args, torch):
     """The 48 instances in the mixed form: one batch handle per grid class
     (every kernel advances the whole class in one launch, graph-replayed
-    steps, autotuned tiles), the classes on their own streams and
+    steps), the classes on their own streams and
     overlapping; against the same instances run one at a time in the plain
     FP64 form."""
     from lesgo_gb300.solver import LesgoGPU
@@ -541,7 +541,7 @@ def run_ours(args):
         "vs_baseline": None, "dtype": "f32 (f64 pressure solve, wall law, step constants)",
         "data": "synthetic (seeded log-law + noise IC)",
         "config": {"workload": WORKLOAD_DESC + "; mixed form (FP32 bulk, FP64 Poisson), one batch per grid "
-                               "class, graph-replayed steps, autotuned tiles",
+                               "class, graph-replayed steps",
                    "instances": batched["instances"], "grids": batched["grids"],
                    "sgs": "Lagrangian scale-dependent, every 5 steps", "dt": 2e-4,
                    "vs_fp64_plain_one_at_a_time": batched["ratio_vs_fp64_one_at_a_time"],

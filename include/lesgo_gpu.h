@@ -373,7 +373,9 @@ int lesgo_gpu_time_step(lesgo_handle_t* h, int id, double* dt);
  * step constants and disk states are copied aside on the device first and
  * put back after, so the simulation state is unchanged (tile shapes do not
  * change results); without memory for that copy the passes are timed alone
- * on scratch buffers.  Call it once after the instances are in place. */
+ * on scratch buffers.  A shape that no pass of the handle's step reads (the
+ * register-transform passes have none) is returned as it is, untimed.  Call
+ * it once after the instances are in place. */
 int lesgo_gpu_autotune(lesgo_handle_t* h, int* xtarget, int* ybudget);
 
 /* ---- instrumentation (no reference counterpart; the reference only

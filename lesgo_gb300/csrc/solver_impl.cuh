@@ -942,9 +942,18 @@ class Solver : public SolverBase {
   // a step with the dynamic update run eagerly per candidate, and the copy is
   // put back, so the simulation state is unchanged (tile shapes do not change
   // results).  Without memory for the copy, the passes are timed alone on
-  // scratch buffers instead.
+  // scratch buffers instead.  A shape that no launch of the step reads (the
+  // register passes have none) stays as it is: timing it would only pick one
+  // by the clock's noise.
+  bool tunes_x() const { return !rx_tw_ || !rxb_tw_; }
+  bool tunes_y() const { return !kRf<A> || !ry_twn_; }
   void autotune(int* xt_out, int* yb_out) override {
     need_active();
+    if (tunes_x() || tunes_y()) tune();
+    if (xt_out) *xt_out = xtarget_;
+    if (yb_out) *yb_out = (int)ybudget_;
+  }
+  void tune() {
     const size_t fbytes = (size_t)nfield_ * sizeof(R);
     const size_t sbytes = (size_t)SC_N * cap_ * sizeof(double);
     const size_t tbytes = kp_.turbines ? 3 * (size_t)th_.n * sizeof(double) : 0;
@@ -973,10 +982,11 @@ class Solver : public SolverBase {
       // handles' and single timings vary by about that much
       struct Cand { int xt; size_t yb; float ms; };
       std::vector<Cand> cands;
-      for (int xt : {1024, 2048, 4096})
-        for (size_t yb : {(size_t)32768, (size_t)49152, (size_t)65536, (size_t)112640}) cands.push_back({xt, yb, 1e30f});
       const int x0 = xtarget_;
       const size_t y0 = ybudget_;
+      for (int xt : tunes_x() ? std::vector<int>{1024, 2048, 4096} : std::vector<int>{x0})
+        for (size_t yb : tunes_y() ? std::vector<size_t>{32768, 49152, 65536, 112640} : std::vector<size_t>{y0})
+          cands.push_back({xt, yb, 1e30f});
       for (int round = 0; round < 3; ++round)
         for (auto& cd : cands) {
           xtarget_ = cd.xt;
@@ -1008,8 +1018,6 @@ class Solver : public SolverBase {
       cudaFree(snap);
     }
     graphs_clear();   // tile shapes are part of the captured launches
-    if (xt_out) *xt_out = xtarget_;
-    if (yb_out) *yb_out = (int)ybudget_;
   }
   // The fallback: the three pass kinds timed alone on scratch buffers (6
   // fields forward from the fields and inverse into the 3/2-grid scratch;
@@ -1033,7 +1041,7 @@ class Solver : public SolverBase {
     const R sc = (R)(1.0 / ((double)d_.nx * ny));
     float best = 1e30f;
     int best_x = xtarget_;
-    for (int xt : {1024, 2048, 4096}) {
+    for (int xt : tunes_x() ? std::vector<int>{1024, 2048, 4096} : std::vector<int>()) {
       xtarget_ = xt;
       const float ms = timed([&] {
         SrcFields<R, 6> src{{F_[LESGO_U], F_[LESGO_V], F_[LESGO_W], F_[LESGO_DUDX], F_[LESGO_DUDY], F_[LESGO_DUDZ]},
@@ -1049,7 +1057,7 @@ class Solver : public SolverBase {
     xtarget_ = best_x;
     best = 1e30f;
     size_t best_y = ybudget_;
-    for (size_t yb : {(size_t)32768, (size_t)49152, (size_t)65536, (size_t)112640}) {
+    for (size_t yb : tunes_y() ? std::vector<size_t>{32768, 49152, 65536, 112640} : std::vector<size_t>()) {
       ybudget_ = yb;
       const float ms = timed([&] {
         ypass_lin<1, 3, true, true, T2, T2>(specA_, 0, 1, nz, ny, specB_, ny, nz, 3, ROW_SAME,

@@ -109,3 +109,18 @@ def test_autotune_keeps_state(built_lib, monkeypatch):
         assert np.array_equal(a.get(f)[1:a.nz, :, :48], b.get(f)[1:b.nz, :, :48]), f
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("precision,nx,ny,x,y", [("mixed", 48, 32, False, False), ("mixed", 64, 16, False, True),
+                                                 ("mixed", 24, 32, True, False), ("fp64", 48, 32, True, False),
+                                                 ("fp64dw", 48, 32, True, True)])
+def test_autotune_leaves_shapes_that_nothing_reads(built_lib, monkeypatch, precision, nx, ny, x, y):
+    """Only the tile shapes of passes that the step launches are tuned (x: the
+    x or 3/2-grid row passes are run-time ones; y: some y pass is)."""
+    monkeypatch.setenv("LESGO_XTARGET", "512")
+    monkeypatch.setenv("LESGO_YBUDGET", "20000")
+    g = handle(nx=nx, ny=ny, Nz=12, precision=precision)
+    g.init_ic(1)
+    cfg = g.autotune()
+    assert (cfg["xtarget"] == 512) != x and (cfg["ybudget"] == 20000) != y, cfg
+    g.close()
