@@ -38,11 +38,21 @@ __host__ __device__ inline long long conv_rows_smem_elems(int rt, int ls, int K)
   return 4LL * 6 * rt * ls + conv_rows_stage_elems(rt, K);
 }
 
+// The lines' complex type.  Double-word: the component-wise operators.  The
+// packed ones run on one half of the FMA pipe only and their register pairs
+// take moves (128x128x64, ncu, against component-wise: heavy half 79 M
+// instructions against 75 M, other half 8 M against 72 M, ALU 54 M against 22
+// M), which at a quarter of the warps resident costs more than the issue
+// slots saved: 557 us at 128^3 against 520, 292 against 273 at 128x128x64, 98
+// against 92 at 96x64x48, 1682 against 1630 at 256x256x96.
+template <typename R> using RowsC = std::conditional_t<std::is_same<R, df64>::value, dfs, cplx<R>>;
+
 // R is the transforms' arithmetic type; the products are formed in it too.
 template <typename R>
-__global__ void __launch_bounds__(256) k_convec_rows(ConvRowsGeom g, FftPlan<R> plan, const cplx<R>* __restrict__ in,
-                                                     cplx<R>* __restrict__ out, R c) {
-  using T2 = cplx<R>;
+__global__ void __launch_bounds__(256) k_convec_rows(ConvRowsGeom g, FftPlan<R> plan, const RowsC<R>* __restrict__ in,
+                                                     RowsC<R>* __restrict__ out, R c) {
+  using T2 = RowsC<R>;
+  const T2* rtw = reinterpret_cast<const T2*>(plan.rtw);
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T2* base = reinterpret_cast<T2*>(smem_raw);
   const int H = g.M / 2;
@@ -126,7 +136,7 @@ __global__ void __launch_bounds__(256) k_convec_rows(ConvRowsGeom g, FftPlan<R> 
         const T2 xm = (k > 0 && km < g.K) ? src[km] : czero<T2>();
         const T2 a = cadd_conj(xk, xm);
         const T2 b = csub_conj(xk, xm);
-        z = cadd(a, mul_pi(cmulconj(b, ldt(plan.rtw + k))));
+        z = cadd(a, mul_pi(cmulconj(b, ldt(rtw + k))));
       }
       A[l * g.ls + k] = z;
     }
@@ -212,7 +222,7 @@ __global__ void __launch_bounds__(256) k_convec_rows(ConvRowsGeom g, FftPlan<R> 
       const T2 a = cadd_conj(zk, zm);
       const T2 b = csub_conj(zk, zm);
       out[(long long)f * g.out_fs + (orow + row0 + r) * g.K + kk] =
-          phalf(cadd(a, mul_mi(cmul(ldt(plan.rtw + kk), b))));
+          phalf(cadd(a, mul_mi(cmul(ldt(rtw + kk), b))));
     }
     __syncthreads();
   }

@@ -37,6 +37,14 @@ struct alignas(16) dfc {
   df64 x, y;
 };
 
+// The same value, computed with df64's operators component by component; the
+// packed forms below are dfc's.  For k_convec_rows, which is faster so.
+struct alignas(16) dfs {
+  df64 x, y;
+  dfs() = default;
+  __device__ __forceinline__ dfs(dfc c) : x(c.x), y(c.y) {}
+};
+
 template <typename R> struct CplxOf;
 template <> struct CplxOf<double> { using T = double2; };
 template <> struct CplxOf<float> { using T = float2; };
@@ -108,6 +116,7 @@ __device__ __forceinline__ dfc ldt(const dfc* p) {
   const float4 v = __ldg(reinterpret_cast<const float4*>(p));
   return dfc{df64{v.x, v.y}, df64{v.z, v.w}};
 }
+__device__ __forceinline__ dfs ldt(const dfs* p) { return ldt(reinterpret_cast<const dfc*>(p)); }
 
 template <typename T2> __device__ __forceinline__ T2 cadd(T2 a, T2 b) { return mkc(a.x + b.x, a.y + b.y); }
 template <typename T2> __device__ __forceinline__ T2 csub(T2 a, T2 b) { return mkc(a.x - b.x, a.y - b.y); }
@@ -138,7 +147,8 @@ template <typename T2> __device__ __forceinline__ T2 cmulconj(T2 a, T2 b) {  // 
 // above would apply twice).  The double-word form's transforms issue 65 to
 // 70 % FP32 instructions; packed, half as many (the 42-field Lagrangian
 // inverse at 128^3 2.03 -> 1.52 ms, the other x passes 5 %, the y passes the
-// same: the FP32 pipe bounds those).
+// same: the FP32 pipe bounds those; the one-pass 3/2-grid rows lose, and have
+// dfs).
 __device__ __forceinline__ float2 df_hi(dfc a) { return make_float2(a.x.hi, a.y.hi); }
 __device__ __forceinline__ float2 df_lo(dfc a) { return make_float2(a.x.lo, a.y.lo); }
 __device__ __forceinline__ dfc df_pack(float2 h, float2 l) { return dfc{df64{h.x, l.x}, df64{h.y, l.y}}; }
@@ -358,7 +368,7 @@ __device__ __forceinline__ void lines_stage(const T2* a, T2* b, int nl, int ls, 
 // Double-word plans use radix 4, 3 and 2 only: their butterflies are long,
 // and leaving radix 8 out of them keeps the kernels' code (and its compile
 // time) small at the same arithmetic per point.
-template <typename T2> constexpr bool kRadix8 = !std::is_same<T2, dfc>::value;
+template <typename T2> constexpr bool kRadix8 = !std::is_same<T2, dfc>::value && !std::is_same<T2, dfs>::value;
 
 template <typename T2, bool INV, bool FIRST>
 __device__ __forceinline__ void lines_stage_r(int Rr, const T2* a, T2* b, int nl, int ls, int nb, int Ns,
@@ -381,16 +391,17 @@ __device__ __forceinline__ void lines_stage_r(int Rr, const T2* a, T2* b, int nl
 // passed by value (registers): the plan lives in the kernel's parameter
 // block, and a reference into it with the run-time stage index would be
 // re-read through the constant path inside the butterfly loop.
-template <typename R, bool INV>
-__device__ cplx<R>* fft_lines(cplx<R>* a, cplx<R>* b, int nl, int ls, const FastDiv fnl, const FftPlan<R>& p) {
+template <typename R, bool INV, typename T2>
+__device__ T2* fft_lines(T2* a, T2* b, int nl, int ls, const FastDiv fnl, const FftPlan<R>& p) {
+  const T2* stw = reinterpret_cast<const T2*>(p.stw);
   for (int s = 0; s < p.nf; ++s) {
     const int nb = p.nbs[s], Ns = p.nss[s];
     if (s == 0)
-      lines_stage_r<cplx<R>, INV, true>(p.radix[s], a, b, nl, ls, nb, Ns, fnl, p.fns[s], p.stw);
+      lines_stage_r<T2, INV, true>(p.radix[s], a, b, nl, ls, nb, Ns, fnl, p.fns[s], stw);
     else
-      lines_stage_r<cplx<R>, INV, false>(p.radix[s], a, b, nl, ls, nb, Ns, fnl, p.fns[s], p.stw + p.two[s]);
+      lines_stage_r<T2, INV, false>(p.radix[s], a, b, nl, ls, nb, Ns, fnl, p.fns[s], stw + p.two[s]);
     __syncthreads();
-    cplx<R>* tmp = a; a = b; b = tmp;
+    T2* tmp = a; a = b; b = tmp;
   }
   return a;
 }

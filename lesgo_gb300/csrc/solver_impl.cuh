@@ -2362,7 +2362,8 @@ class Solver : public SolverBase {
     g.cz = (d_.nz + best_n - 1) / best_n;
     dim3 grid((unsigned)((d_.ny2 + rt - 1) / rt), (unsigned)((d_.nz + g.cz - 1) / g.cz), (unsigned)kp_.ninst);
     pre();
-    kern<<<grid, 256, smem, st_>>>(g, pxb_, cvB_, cvA_, cb);
+    kern<<<grid, 256, smem, st_>>>(g, pxb_, reinterpret_cast<const RowsC<A>*>(cvB_),
+                                   reinterpret_cast<RowsC<A>*>(cvA_), cb);
     post("convec.rows", 9.0 * vol1_b_ * kp_.ninst * sizeof(T2));
   }
   void convec_part2(bool fused) {
