@@ -78,7 +78,7 @@ def parse():
                     "ensemble)")
     ap.add_argument("--val-members", type=int, default=None, help="realisations per side (default 3 for B, 1 for C)")
     ap.add_argument("--xdft-compare", action="store_true", help="the forward x transforms as tensor-core GEMMs "
-                    "(LESGO_XDFT=1) against the radix kernels: per-stage and whole-step times")
+                    "(LESGO_XDFT=1) against the default x passes: per-stage and whole-step times")
     ap.add_argument("--only-class", default=None, help="run only the ensemble's instances of one grid class, "
                     "e.g. 96x96x64 (each class is an independent batch: used to profile its launches alone)")
     return ap.parse_args()
@@ -706,8 +706,8 @@ def run_validate(args):
 
 def run_xdft_compare(args):
     """The forward x transforms as tensor-core GEMMs (k_xdft_tc: three-pass
-    TF32 splitting, FP32 accuracy; LESGO_XDFT=1) against the radix kernels
-    (k_xfwd), in the mixed form: the x-forward stages' CUDA-event times and
+    TF32 splitting, FP32 accuracy; LESGO_XDFT=1) against the default x
+    passes (k_rx_fwd at listed lengths, else k_xfwd), in the mixed form: the x-forward stages' CUDA-event times and
     achieved algorithmic GB/s, and the whole step's device time, for one
     128^3 instance and for the 48-instance ensemble.  Both arms run the same
     instances from the same seeds; the tiles are autotuned per arm."""

@@ -30,7 +30,7 @@ void ry_spec(const RyArgs<A, cplx<A>, double2>& a, int ny, int nlev, int nf, cud
 template <typename A>
 void ry_phys(bool grad, const RyArgs<A, double2, cplx<A>>& a, int ny, int nlev, cudaStream_t st);
 
-// cz = 0: chosen from the launch's waves
+// g.cz, the levels per block, is set here from the launch's waves
 template <typename A>
 void rx_rows(RxRowsGeom<A> g, int H, int ninst, const cplx<A>* in, cplx<A>* out, A c, cudaStream_t st);
 

@@ -17,16 +17,15 @@
 
 namespace lesgo {
 
-// cos and sin of 2 pi m / R for the composite butterflies' inner twiddles.
+// cos and sin of 2 pi m / R for the composite butterflies' inner twiddles
+// (the 9- and 16-point ones; the others are prime-factor products).
 __host__ __device__ constexpr double root_cos(int m, int R) {
   m %= R;
   if (2 * m > R) m = R - m;
   const int t = 144 * m / R;   // in units of 2.5 degrees (R divides 144)
-  return t == 0 ? 1.0 : t == 4 ? 0.98480775301220805937 : t == 6 ? 0.96592582628906828675
-       : t == 8 ? 0.93969262078590838405 : t == 9 ? 0.92387953251128675613 : t == 12 ? 0.86602540378443864676
+  return t == 4 ? 0.98480775301220805937 : t == 8 ? 0.93969262078590838405 : t == 9 ? 0.92387953251128675613
        : t == 16 ? 0.76604444311897803520 : t == 18 ? 0.70710678118654752440 : t == 20 ? 0.64278760968653932632
-       : t == 24 ? 0.5 : t == 27 ? 0.38268343236508977173 : t == 28 ? 0.34202014332566873304
-       : t == 30 ? 0.25881904510252076235 : t == 32 ? 0.17364817766693034885 : t == 36 ? 0.0
+       : t == 27 ? 0.38268343236508977173 : t == 28 ? 0.34202014332566873304 : t == 32 ? 0.17364817766693034885
        : -root_cos(72 - t, 144);
 }
 __host__ __device__ constexpr double root_sin(int m, int R) {
@@ -168,7 +167,8 @@ template <typename T2, typename A> __device__ __forceinline__ T2 add_ik(T2 a, A 
 }
 
 // The factors of a length, chosen at compile time from a list; the host
-// asks the same list (rf_factors) to build the twiddle table.
+// asks the same list (rx_factors, ry_factors, rxb_factors) to build the
+// twiddle table.
 template <int A, int B> struct Len {
   static constexpr int R1 = A, R2 = B, N = A * B;
 };

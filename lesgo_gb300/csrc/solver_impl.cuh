@@ -2310,8 +2310,8 @@ class Solver : public SolverBase {
   void convec_rows(A cb) {
     if constexpr (kRfRows<A>) {
       if (rxb_tw_) {
-        RxRowsGeom<A> rg;
-        rg.ny2 = d_.ny2; rg.nz = d_.nz; rg.cz = 0; rg.err = err_ + 1;
+        RxRowsGeom<A> rg{};
+        rg.ny2 = d_.ny2; rg.nz = d_.nz; rg.err = err_ + 1;
         rg.in_fs = rg.out_fs = vol1_b_ * kp_.ninst;
         rg.tw = rxb_tw_; rg.rtw = pxb_.rtw;
         pre();
