@@ -548,7 +548,7 @@ def run_ours(args):
                    "fp64_plain_one_at_a_time": batched["fp64_one_at_a_time"],
                    "vs_fp64dw_one_at_a_time": batched["ratio_vs_fp64dw_one_at_a_time"],
                    "fp64dw_one_at_a_time": batched["fp64dw_one_at_a_time"],
-                   "profile_error": "mean profile <= 1e-2 against FP64 (128^3: 2.6e-4; wind farm: 2.6e-5)",
+                   "profile_error": "mean profile <= 1e-2 against FP64 (128^3: 4.9e-4; wind farm: 6.5e-6)",
                    "parallelism": f"replicas x{world}" if world > 1 else "1 GPU",
                    "l2": "working set > L2 (about 3 GB of fields)"},
         "e2e": {"value": e2e["value"], "unit": UNIT, "h2d_bytes_per_step": e2e["h2d"], "d2h_bytes_per_step": e2e["d2h"]},

@@ -21,7 +21,10 @@
 // % active, ncu): each row holds 8 KB of exchange lines and copies.  Mixed
 // form, us per launch against k_convec_rows (and the 9 spectra at the copy
 // bandwidth): 128^3 70 (141; 17), 256x256x192 353 (841; 101), 6 x 108x72x30
-// 68 (11), 48^3 16.5 (18.5; 1).  Measured and dropped: one field per
+// 68 (11), 48^3 16.5 (18.5; 1).  Slower where few blocks leave the longer
+// chain of a level exposed, in a step that is shorter all the same: one
+// instance of 64x16x32 17.4 (14.3), of 64x48x24 17.8 (15.1), their whole
+// steps 95.6 us (152) and 82 (177).  Measured and dropped: one field per
 // exchange with 12 barriers a level and the spectra read in place (95 us at
 // 128^3, 855 us at 256x256x192).
 #pragma once
