@@ -58,3 +58,20 @@ def test_boundaries(built_lib, precision, bc, grid):
 def test_moving_bottom_wall(built_lib, precision, grid):
     """The no-slip wall's velocity is taken off the mean mode of u."""
     check(precision, grid, dict(lbc_mom=1, molec=True, ubot=3.0), grid == (48, 36, 12) and precision != "fp64dw")
+
+
+NX = [32, 36, 48, 64, 72, 96, 108, 128, 144, 192, 216, 256]
+NY = [24, 32, 36, 48, 54, 64, 72, 96, 108, 128, 144, 192, 216, 256]
+
+
+@pytest.mark.parametrize("nx,ny", [(NX[i % len(NX)], ny) for i, ny in enumerate(NY)])
+def test_listed_lengths_take_the_register_passes(built_lib, nx, ny):
+    """(Where they did not, a comparison with the run-time passes would be
+    one of these with themselves.)"""
+    from lesgo_gb300.solver import LesgoGPU
+    g = LesgoGPU(nx=nx, ny=ny, Nz=4, precision="mixed")
+    g.init_ic(1)
+    g.profile(True)
+    g.step(1)
+    assert "convec.ypass_vpad" in g.profile_report()
+    g.close()
